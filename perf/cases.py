@@ -193,3 +193,18 @@ def tolerance(case):
     if "fp16" in types:
         return {"rel": 1.5e-3}
     return {"rel": 5e-7}
+
+
+def exact(case, seed):
+    """The scaled gradients (cast), the gradients themselves (a group of one rank) or their mean at every rank, in 64
+    bits.  The wire's rounding is part of what a group of one rank returns; elsewhere it is the implementation's error."""
+    count, dtype = case["count"], case["dtype"]
+    if case["entry"] == "cast":
+        return _gradients(count, dtype, seed, 0).double() * (1.0 / 8)
+    if case["entry"] == "c10d":
+        return _gradients(count, dtype, seed, 0).to(DTYPES[case["wire"]]).double()
+    mean = torch.zeros(count, device="cuda", dtype=torch.float64)
+    for r in range(case["n"]):
+        mean += _gradients(count, dtype, seed, r).double()
+    mean /= case["n"]
+    return [mean] * case["n"]
