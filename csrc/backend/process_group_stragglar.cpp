@@ -356,6 +356,8 @@ void ProcessGroupStragglar::run_program(Side& s, const sar::Program& prog, size_
       P.ops = (const SarOp*)it->second.first;
       P.round_begin = (const uint16_t*)it->second.second;
       P.num_rounds = rt.round_begin.empty() ? 0 : (uint32_t)rt.round_begin.size() - 1;
+      P.num_ops = (uint32_t)rt.ops.size();
+      P.one_device = n == 1;
       P.geom = g; P.rank = me; P.nranks = n; P.participants = c.participants;
       P.epoch_base = epoch; P.scale = scale; P.dtype = dt;
       P.timeout_ns = (uint64_t)(opts_.timeout_s * 1e9);

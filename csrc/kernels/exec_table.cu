@@ -3,6 +3,7 @@
 #include "sar_cuda.h"
 
 #include <cooperative_groups.h>
+#include <cstring>
 
 using namespace sar_dev;
 
@@ -26,42 +27,48 @@ __global__ void __launch_bounds__(simta::kThreads, 1) sar_exec_simta_kernel(cons
 
 // All ranks of a collective in one launch on one device (tests, profiling).
 // Blocks of different ranks wait on one another, so they must be co-resident:
-// launched cooperatively.
-template <typename T>
-__global__ void __launch_bounds__(512, 1) sar_emul_simt_kernel(const SarLaunchParams* params, int blocks_per_rank) {
-  __shared__ SarLaunchParams P;
-  const int r = blockIdx.x / blocks_per_rank;
+// launched cooperatively.  The parameters come with the launch; every block puts
+// its rank's view of them together in shared memory.
+__device__ __forceinline__ void load_rank_params(const SarEmulParams& E, int r, SarLaunchParams& P) {
   for (uint32_t i = threadIdx.x; i < sizeof(SarLaunchParams) / 4; i += blockDim.x)
-    reinterpret_cast<uint32_t*>(&P)[i] = reinterpret_cast<const uint32_t*>(params + r)[i];
+    reinterpret_cast<uint32_t*>(&P)[i] = reinterpret_cast<const uint32_t*>(&E.common)[i];
   __syncthreads();
+  if (threadIdx.x == 0) {
+    const SarEmulRank& R = E.rank[r];
+    P.rank = r;
+    P.ops = R.ops; P.round_begin = R.round_begin; P.num_rounds = R.num_rounds; P.num_ops = R.num_ops;
+    P.status = R.status; P.trace = R.trace; P.delay_ns = R.delay_ns;
+    P.user_in = R.user_in; P.user_out = R.user_out;
+    for (int c = 0; c < SAR_MAX_CHUNKS; ++c) P.final_ver[c] = R.final_ver[c];
+  }
+  __syncthreads();
+}
+static_assert(sizeof(SarLaunchParams) % 4 == 0, "params are copied word by word");
+
+template <typename T>
+__global__ void __launch_bounds__(512, 1) sar_emul_simt_kernel(const __grid_constant__ SarEmulParams E, int blocks_per_rank) {
+  __shared__ SarLaunchParams P;
+  load_rank_params(E, blockIdx.x / blocks_per_rank, P);
   if (!(P.participants >> P.rank & 1)) return;
   run_rank_simt<T>(P, blockIdx.x % blocks_per_rank, blocks_per_rank);
 }
 
 template <typename T>
-__global__ void __launch_bounds__(simta::kThreads, 1) sar_emul_simta_kernel(const SarLaunchParams* params, int blocks_per_rank) {
+__global__ void __launch_bounds__(simta::kThreads, 1) sar_emul_simta_kernel(const __grid_constant__ SarEmulParams E, int blocks_per_rank) {
   __shared__ SarLaunchParams P;
   __shared__ simta::Shared S;
-  const int r = blockIdx.x / blocks_per_rank;
-  for (uint32_t i = threadIdx.x; i < sizeof(SarLaunchParams) / 4; i += blockDim.x)
-    reinterpret_cast<uint32_t*>(&P)[i] = reinterpret_cast<const uint32_t*>(params + r)[i];
-  __syncthreads();
+  load_rank_params(E, blockIdx.x / blocks_per_rank, P);
   if (!(P.participants >> P.rank & 1)) return;
   run_rank_simta<T>(P, blockIdx.x % blocks_per_rank, blocks_per_rank, S);
 }
 
 template <typename T>
-__global__ void __launch_bounds__(tma::kThreads, 1) sar_emul_tma_kernel(const SarLaunchParams* params, int blocks_per_rank) {
+__global__ void __launch_bounds__(tma::kThreads, 1) sar_emul_tma_kernel(const __grid_constant__ SarEmulParams E, int blocks_per_rank) {
   __shared__ SarLaunchParams P;
-  const int r = blockIdx.x / blocks_per_rank;
-  for (uint32_t i = threadIdx.x; i < sizeof(SarLaunchParams) / 4; i += blockDim.x)
-    reinterpret_cast<uint32_t*>(&P)[i] = reinterpret_cast<const uint32_t*>(params + r)[i];
-  __syncthreads();
+  load_rank_params(E, blockIdx.x / blocks_per_rank, P);
   if (!(P.participants >> P.rank & 1)) return;
   run_rank_tma<T>(P, blockIdx.x % blocks_per_rank, blocks_per_rank, *reinterpret_cast<tma::Shared*>(sar_smem));
 }
-
-static_assert(sizeof(SarLaunchParams) % 4 == 0, "params are copied word by word");
 
 __global__ void sar_barrier_kernel(SarDevComm comm, int rank, int nranks, uint32_t participants, uint32_t epoch,
                                    uint64_t timeout_ns, uint32_t* status) {
@@ -70,6 +77,7 @@ __global__ void sar_barrier_kernel(SarDevComm comm, int rank, int nranks, uint32
   w.deadline = globaltimer() + timeout_ns;
   w.abort_flag = &comm.ctrl[rank]->abort_flag;
   w.status = status;
+  w.one_device = false;
   fence_sys();
   st_release_sys(&comm.ctrl[rank]->arrival, epoch);
   for (int r = 0; r < nranks; ++r) {
@@ -87,6 +95,7 @@ __global__ void sar_signal_wait_kernel(uint32_t* set_ptr, uint32_t set_val, cons
     w.deadline = globaltimer() + timeout_ns;
     w.abort_flag = abort_flag;
     w.status = status;
+    w.one_device = false;
     wait_word(wait_ptr, wait_val, w, SAR_TIMEOUT_FLAG);
   }
 }
@@ -302,13 +311,24 @@ int sar_cuda_max_emulated_blocks(int dtype, int path, int threads) {
   return sms * per_sm;
 }
 
-int sar_cuda_launch_emulated(const SarLaunchParams* d_params, int n, int dtype, int path, int blocks_per_rank,
-                             int threads, void* stream) {
+int sar_cuda_launch_emulated(const SarLaunchParams* params, int n, int path, int blocks_per_rank, int threads, void* stream) {
+  if (n < 1 || n > SAR_MAX_RANKS) return (int)cudaErrorInvalidValue;
   if (blocks_per_rank <= 0) blocks_per_rank = 4;
   cudaStream_t st = (cudaStream_t)stream;
-  return with_dtype(dtype, [&](auto tag) -> int {
+  SarEmulParams E;
+  E.common = params[0];
+  memset(E.rank, 0, sizeof E.rank);
+  for (int r = 0; r < n; ++r) {
+    const SarLaunchParams& P = params[r];
+    SarEmulRank& R = E.rank[r];
+    R.ops = P.ops; R.round_begin = P.round_begin; R.num_rounds = P.num_rounds; R.num_ops = P.num_ops;
+    R.status = P.status; R.trace = P.trace; R.delay_ns = P.delay_ns;
+    R.user_in = P.user_in; R.user_out = P.user_out;
+    memcpy(R.final_ver, P.final_ver, sizeof R.final_ver);
+  }
+  return with_dtype(E.common.dtype, [&](auto tag) -> int {
     using T = decltype(tag);
-    void* args[] = {(void*)&d_params, (void*)&blocks_per_rank};
+    void* args[] = {(void*)&E, (void*)&blocks_per_rank};
     if (path == SAR_PATH_TMA) {
       int e = allow_smem(sar_emul_tma_kernel<T>, sizeof(tma::Shared));
       if (e) return e;

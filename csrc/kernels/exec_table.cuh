@@ -58,6 +58,12 @@ __device__ __forceinline__ void st_relaxed_sys(uint32_t* p, uint32_t v) {
   asm volatile("st.relaxed.sys.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 __device__ __forceinline__ void fence_sys() { asm volatile("fence.acq_rel.sys;" ::: "memory"); }
+// Orders what this thread has seen and written for the other ranks: system scope between devices, device scope when
+// every rank of the launch runs on this device (SarLaunchParams::one_device; the fence is then answered by L2).
+__device__ __forceinline__ void fence_ranks(bool one_device) {
+  if (one_device) asm volatile("fence.acq_rel.gpu;" ::: "memory");
+  else fence_sys();
+}
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async;" ::: "memory"); }
 // 16-byte load that is coherent at system scope (never served from a stale L1 line)
 __device__ __forceinline__ uint4 ld_vec_sys(const void* p) {
@@ -171,6 +177,7 @@ struct WaitCtx {
   uint64_t deadline;        // %globaltimer value after which waits give up
   uint32_t* abort_flag;     // this rank's abort word (local memory)
   uint32_t* status;
+  bool one_device;          // scope of the fences (see fence_ranks)
 };
 __device__ __forceinline__ void record_failure(const WaitCtx& w, uint32_t code) {
   if (w.status) atomicCAS(w.status, 0u, code);
@@ -179,10 +186,9 @@ __device__ __forceinline__ void record_failure(const WaitCtx& w, uint32_t code) 
 }
 // Spin until *p reaches target; false on abort or deadline (failure recorded).
 __device__ __noinline__ bool wait_word(const uint32_t* p, uint32_t target, const WaitCtx& w, uint32_t fail_code) {
-  if (sar_reached(ld_acquire_sys(p), target)) return true;
   uint32_t ns = 20;
   for (uint64_t it = 0;; ++it) {
-    if (sar_reached(ld_acquire_sys(p), target)) return true;
+    if (sar_reached(ld_relaxed_sys(p), target)) { fence_ranks(w.one_device); return true; }   // acquire
     if ((it & 15) == 15) {
       if (*(volatile uint32_t*)w.abort_flag) return false;
       if (globaltimer() > w.deadline) { record_failure(w, fail_code); return false; }
@@ -205,7 +211,7 @@ __device__ __noinline__ uint32_t wait_mirrors(const uint32_t* words, uint32_t ma
     uint32_t missing = 0;
 #pragma unroll
     for (int r = 0; r < SAR_MAX_RANKS; ++r) if (!sar_reached(v[r], target)) missing |= 1u << r;
-    if (!missing) { fence_sys(); return 0; }   // acquire: what the announcers wrote before is visible now
+    if (!missing) { fence_ranks(w.one_device); return 0; }   // acquire: what the announcers wrote before is visible now
     if ((it & 15) == 15) {
       if (*(volatile uint32_t*)w.abort_flag) return missing;
       if (globaltimer() > w.deadline) { record_failure(w, fail_code); return missing; }
@@ -235,7 +241,9 @@ struct OpGeom {
 };
 struct RoundGeom { uint32_t op_begin, m, max_tiles, pad; };
 struct TableGeom {
+  SarOp ops[SAR_MAX_OPS];               // the rank's table itself: read for every piece by every role of the block
   OpGeom op[SAR_MAX_OPS];
+  uint16_t round_begin[SAR_MAX_ROUNDS + 1];
   RoundGeom round[2][SAR_MAX_ROUNDS];   // per lane
   SarOp stage_op[2];                    // pseudo ops of staged mode: [0] SAR_STAGE_IN, [1] SAR_STAGE_OUT
   uint32_t num_rounds;
@@ -258,34 +266,37 @@ __device__ __forceinline__ uint32_t staging_blocks(const SarLaunchParams& P, uin
 }
 
 // All threads of the block; ends with a block barrier.
+//
+// Bound by latency, on the path of every collective: the table is fetched with one round of coalesced loads (ops and
+// round offsets together), and everything derived from it is computed by as many threads as there are ops or rounds.
+// Walking the ops in global memory with one thread instead cost a trip to L2 per op, and every later look at an op
+// another one, because the acquiring fences of the waits empty L1.
+// Eight ranks on one device, 4 KiB: 38 -> 19 us in the kernel (rsag, bulk-copy path), 34 -> 15 us (simt); of that the
+// fences at device scope and the flag polls kept in registers (wait_item_ready) are about half.
 __device__ void resolve_table(const SarLaunchParams& P, TableGeom& G, uint32_t nblocks) {
   const uint32_t nrounds = P.num_rounds < SAR_MAX_ROUNDS ? P.num_rounds : SAR_MAX_ROUNDS;
-  const uint32_t nops = nrounds ? P.round_begin[nrounds] : 0;
-  for (uint32_t o = threadIdx.x; o < nops && o < SAR_MAX_OPS; o += blockDim.x) {
-    const SarOp op = P.ops[o];
+  const uint32_t nops = nrounds ? (P.num_ops < SAR_MAX_OPS ? P.num_ops : SAR_MAX_OPS) : 0;
+  for (uint32_t i = threadIdx.x; i < nops * (sizeof(SarOp) / 4); i += blockDim.x)
+    reinterpret_cast<uint32_t*>(G.ops)[i] = reinterpret_cast<const uint32_t*>(P.ops)[i];
+  if (nrounds)
+    for (uint32_t r = threadIdx.x; r <= nrounds; r += blockDim.x) G.round_begin[r] = P.round_begin[r];
+  __syncthreads();
+  bool second_lane = false;
+  for (uint32_t o = threadIdx.x; o < nops; o += blockDim.x) {
+    const SarOp& op = G.ops[o];
     uint32_t t0, t1;
-    sar_part_range(sar_chunk_tiles(P.geom, op.chunk), op.part, op.parts, &t0, &t1);
-    const uint64_t cb = sar_chunk_begin(P.geom, op.chunk);
+    const uint64_t cb = sar_chunk_begin(P.geom, op.chunk), ce = sar_chunk_begin(P.geom, op.chunk + 1u);
+    sar_part_range((uint32_t)((ce - cb + P.geom.tile_elems - 1) / P.geom.tile_elems), op.part, op.parts, &t0, &t1);
     G.op[o].elem0 = cb + (uint64_t)t0 * P.geom.tile_elems;
-    G.op[o].elem_end = cb + sar_chunk_len(P.geom, op.chunk);
+    G.op[o].elem_end = ce;
     G.op[o].ntiles = t1 - t0;
     G.op[o].tile0 = t0;
+    second_lane = second_lane || op.lane != 0;
   }
-  if (threadIdx.x == 0 && P.gate_rounds) {
-    uint32_t items[SAR_GATE_ALL_DONE];
-    for (uint32_t r = 0; r < SAR_GATE_ALL_DONE; ++r) items[r] = 0;
-    for (uint32_t o = 0; o < nops && o < SAR_MAX_OPS; ++o) {
-      const SarOp op = P.ops[o];
-      if (op.round < SAR_GATE_ALL_DONE) items[op.round] += sar_op_tiles(P.geom, op);
-    }
-    G.round_prefix[0] = 0;
-    for (uint32_t r = 0; r < SAR_GATE_ALL_DONE; ++r) G.round_prefix[r + 1] = G.round_prefix[r] + items[r];
-  }
+  const uint32_t table_lanes = __syncthreads_or(second_lane) ? 2u : 1u;
+  uint32_t lanes, lane, lb, lnb;
+  sar_lane_of_block(0, nblocks - staging_blocks(P, nblocks), table_lanes, P.lane1_eighths, &lanes, &lane, &lb, &lnb);
   if (threadIdx.x == 0) {
-    uint32_t table_lanes = 1;
-    for (uint32_t o = 0; o < nops && o < SAR_MAX_OPS; ++o) if (P.ops[o].lane) table_lanes = 2;
-    uint32_t lanes, lane, lb, lnb;
-    sar_lane_of_block(0, nblocks - staging_blocks(P, nblocks), table_lanes, P.lane1_eighths, &lanes, &lane, &lb, &lnb);
     G.lanes = lanes;
     G.num_rounds = nrounds;
     for (int k = 0; k < 2; ++k) {
@@ -295,16 +306,22 @@ __device__ void resolve_table(const SarLaunchParams& P, TableGeom& G, uint32_t n
       G.stage_op[k] = z;
     }
   }
-  __syncthreads();
   for (uint32_t r = threadIdx.x; r < nrounds; r += blockDim.x) {
-    const uint32_t ob = P.round_begin[r], oe = P.round_begin[r + 1];
+    const uint32_t ob = G.round_begin[r], oe = G.round_begin[r + 1];
     uint32_t split = oe;                  // one lane: every op of the round
-    if (G.lanes == 2) { split = ob; while (split < oe && P.ops[split].lane == 0) ++split; }
+    if (lanes == 2) { split = ob; while (split < oe && G.ops[split].lane == 0) ++split; }
     for (uint32_t l = 0; l < 2; ++l) {
       const uint32_t b = l == 0 ? ob : split, e = l == 0 ? split : oe;
       uint32_t mx = 0;
       for (uint32_t o = b; o < e; ++o) mx = G.op[o].ntiles > mx ? G.op[o].ntiles : mx;
       G.round[l][r].op_begin = b; G.round[l][r].m = e - b; G.round[l][r].max_tiles = mx;
+    }
+  }
+  if (P.gate_rounds) {
+    for (uint32_t r = threadIdx.x; r <= SAR_GATE_ALL_DONE; r += blockDim.x) {
+      uint32_t before = 0;
+      for (uint32_t o = 0; o < nops; ++o) if (G.ops[o].round < r && G.ops[o].round < SAR_GATE_ALL_DONE) before += G.op[o].ntiles;
+      G.round_prefix[r] = before;
     }
   }
   __syncthreads();
@@ -386,7 +403,7 @@ struct ItemWalker {
           k += nblocks;
           const OpGeom& og = G->op[o];
           if (lt >= og.ntiles) continue;
-          const SarOp* op = P->ops + o;
+          const SarOp* op = G->ops + o;
           const uint64_t e0 = og.elem0 + (uint64_t)lt * P->geom.tile_elems;
           uint64_t e1 = e0 + P->geom.tile_elems;
           if (e1 > og.elem_end) e1 = og.elem_end;
@@ -451,7 +468,7 @@ __device__ __forceinline__ void gate_announce(const SarLaunchParams& P, uint32_t
 }
 // One thread of the rank's block 0, after resolve_table: the rounds before the first one with items are done.
 __device__ __forceinline__ void gate_announce_first(const SarLaunchParams& P, const TableGeom& G) {
-  fence_sys();
+  fence_ranks(P.one_device);
   gate_announce(P, gate_round_for(G, 0, 0));
 }
 // The thread that has just announced an item: counts it, and announces the rounds that this completes.
@@ -461,7 +478,7 @@ __device__ __forceinline__ void gate_item_done(const SarLaunchParams& P, const T
   const uint32_t done = atomicAdd(&me->items_done, 1u) + 1u;
   const uint32_t R = gate_round_for(G, done, P.gate_slack);
   if (R == 0 || *(volatile uint32_t*)&me->announced >= R + 1u) return;
-  fence_sys();   // the items counted so far (by any thread of this rank) are visible before the announcement
+  fence_ranks(P.one_device);   // the items counted so far (by any thread of this rank) are visible before the announcement
   gate_announce(P, R);
 }
 // Bounded wait until every participant has announced round `round` (the words are in this rank's memory).
@@ -473,7 +490,7 @@ __device__ __noinline__ bool wait_gate(const SarLaunchParams& P, uint32_t round,
     bool all = true;
     for (int r = 0; r < P.nranks; ++r)
       if ((P.participants >> r & 1) && ld_relaxed_sys_u64(g + r) < target) all = false;
-    if (all) { fence_sys(); return true; }   // acquire: what the announcers ordered before is visible now
+    if (all) { fence_ranks(w.one_device); return true; }   // acquire: what the announcers ordered before is visible now
     if ((it & 15) == 15) {
       if (*(volatile uint32_t*)w.abort_flag) return false;
       if (globaltimer() > w.deadline) { record_failure(w, SAR_TIMEOUT_FLAG); return false; }
@@ -501,37 +518,41 @@ __device__ bool wait_item_ready(const SarLaunchParams& P, const Item& it, const 
     // a full barrier between rounds: every participant has arrived and every operand is complete
     if (P.gate_slack == 0 && !staged) { *arrived_mask = P.participants; return true; }
   }
+  const int nsrc = op->nsrc;
   {
     uint32_t need = 0;
-    for (int q = 0; q < op->nsrc; ++q) need |= 1u << op->src[q];
+    for (int q = 0; q < nsrc; ++q) need |= 1u << op->src[q];
     need &= ~*arrived_mask;
     if (need) {
       if (wait_mirrors(P.comm.ctrl[P.rank]->arrival_m, need, P.nranks, P.epoch_base, w, SAR_TIMEOUT_ARRIVAL)) return false;
       *arrived_mask |= need;
     }
   }
-  // every flag the item depends on, polled together: the loads of one turn are independent, so waiting for seven
-  // peers' tiles costs one trip over the link per turn, not seven
-  const uint32_t* ptr[SAR_MAX_RANKS + 1];
-  uint32_t want[SAR_MAX_RANKS + 1];
-  int nf = 0;
+  // every flag the item depends on, polled together: the loads of one turn are independent (the loop is unrolled and
+  // the words stay in registers), so waiting for seven peers' tiles costs one trip over the link per turn, not seven
   // (A push names the version it replaces in the destination.  Version 0 there, in staged mode, is the
   // destination's own copy-in of that tile, and whatever is pushed into a slot contains that rank's contribution to
   // the chunk or follows a read of it, both of which waited for that copy-in: the push is ordered after it already.)
-  for (int q = 0; q < op->nsrc; ++q)
-    if (op->src_ver[q] || (staged && op->kind != SAR_PUSH)) {
-      ptr[nf] = P.comm.flags[op->src[q]] + it.fidx; want[nf] = P.epoch_base + op->src_ver[q]; ++nf;
-    }
-  if (op->local_ver || staged) { ptr[nf] = P.comm.flags[P.rank] + it.fidx; want[nf] = P.epoch_base + op->local_ver; ++nf; }
-  if (nf == 0) return true;
-  if (nf == 1) return wait_word(ptr[0], want[0], w, SAR_TIMEOUT_FLAG);
+  const bool own_flag = op->local_ver || staged;
+  const bool zero_flag = staged && op->kind != SAR_PUSH;
+  uint32_t deps = 0;
+  for (int q = 0; q < nsrc; ++q) deps |= (uint32_t)(op->src_ver[q] || zero_flag) << q;
+  if (!deps) {
+    if (!own_flag) return true;
+    return wait_word(P.comm.flags[P.rank] + it.fidx, P.epoch_base + op->local_ver, w, SAR_TIMEOUT_FLAG);
+  }
+  if (deps == 1 && !own_flag) return wait_word(P.comm.flags[op->src[0]] + it.fidx, P.epoch_base + op->src_ver[0], w, SAR_TIMEOUT_FLAG);
   uint32_t ns = 20;
   for (uint64_t turn = 0;; ++turn) {
-    uint32_t v[SAR_MAX_RANKS + 1];
-    for (int i = 0; i < nf; ++i) v[i] = ld_relaxed_sys(ptr[i]);
-    bool all = true;
-    for (int i = 0; i < nf; ++i) all = all && sar_reached(v[i], want[i]);
-    if (all) { fence_sys(); return true; }   // acquire
+    uint32_t v[SAR_MAX_RANKS];
+    const uint32_t mine = own_flag ? ld_relaxed_sys(P.comm.flags[P.rank] + it.fidx) : P.epoch_base + op->local_ver;
+#pragma unroll
+    for (int q = 0; q < SAR_MAX_RANKS; ++q) v[q] = (deps >> q & 1) ? ld_relaxed_sys(P.comm.flags[op->src[q]] + it.fidx) : 0u;
+    bool all = sar_reached(mine, P.epoch_base + op->local_ver);
+#pragma unroll
+    for (int q = 0; q < SAR_MAX_RANKS; ++q)
+      if (deps >> q & 1) all = all && sar_reached(v[q], P.epoch_base + op->src_ver[q]);
+    if (all) { fence_ranks(w.one_device); return true; }   // acquire
     if ((turn & 15) == 15) {
       if (*(volatile uint32_t*)w.abort_flag) return false;
       if (globaltimer() > w.deadline) { record_failure(w, SAR_TIMEOUT_FLAG); return false; }
@@ -831,9 +852,11 @@ __device__ __forceinline__ WaitCtx enter_collective(const SarLaunchParams& P, ui
   w.deadline = globaltimer() + P.timeout_ns;
   w.abort_flag = &P.comm.ctrl[P.rank]->abort_flag;
   w.status = P.status;
+  w.one_device = P.one_device != 0;
   if (block == 0 && threadIdx.x == 0) {
     if (P.trace) P.trace[0] = globaltimer();
-    st_release_sys(&P.comm.ctrl[P.rank]->arrival, P.epoch_base);
+    fence_ranks(w.one_device);
+    st_relaxed_sys(&P.comm.ctrl[P.rank]->arrival, P.epoch_base);
     // the same word into every participant's memory, where its waits look for it
     for (int q = 0; q < P.nranks; ++q)
       if (q != P.rank && (P.participants >> q & 1)) st_relaxed_sys(&P.comm.ctrl[q]->arrival_m[P.rank], P.epoch_base);
@@ -855,8 +878,8 @@ __device__ void leave_collective(const SarLaunchParams& P, const WaitCtx& w, uin
   me->announced = 0;
   __threadfence();
   if (*(volatile uint32_t*)w.abort_flag == 0) {
-    fence_sys();
-    st_release_sys(&me->exited, P.epoch_base);
+    fence_ranks(w.one_device);
+    st_relaxed_sys(&me->exited, P.epoch_base);
     for (int q = 0; q < P.nranks; ++q)
       if (q != P.rank && (P.participants >> q & 1)) st_relaxed_sys(&P.comm.ctrl[q]->exited_m[P.rank], P.epoch_base);
     wait_mirrors(me->exited_m, P.participants & ~(1u << P.rank), P.nranks, P.epoch_base, w, SAR_TIMEOUT_EXIT);
@@ -898,7 +921,7 @@ __device__ void run_rank_simt(const SarLaunchParams& P, uint32_t block, uint32_t
     simt_tile<T, 4>(P, it, threadIdx.x, blockDim.x);
     __syncthreads();   // every store of the tile is issued; s_item may be rewritten
     if (threadIdx.x == 0) {
-      fence_sys();
+      fence_ranks(w.one_device);
       publish_item(P, it.op, it.fidx);
       trace_item_end(P, it.op);
       gate_item_done(P, G, it.op);
@@ -1319,7 +1342,7 @@ __device__ void run_rank_tma(const SarLaunchParams& P, uint32_t block, uint32_t 
       while (head + n != tail && S.pend[(head + n) % kPendRing].seq < landed) ++n;
       if (n) {
         fence_proxy_async_global();   // the tiles were written by bulk copies
-        fence_sys();
+        fence_ranks(w.one_device);
         for (uint32_t i = 0; i < n; ++i) {
           const PendEntry& e = S.pend[(head + i) % kPendRing];
           publish_item(P, e.op, e.fidx);
@@ -1466,7 +1489,7 @@ __device__ void run_rank_simta(const SarLaunchParams& P, uint32_t block, uint32_
       const uint32_t done = ld_acquire_cta(&S.workers_done);
       const uint32_t tail = ld_acquire_cta(&S.pend_tail);
       if (head != tail) {
-        fence_sys();                   // the tiles' stores (ordered before the hand-off) become visible first
+        fence_ranks(w.one_device);     // the tiles' stores (ordered before the hand-off) become visible first
         for (; head != tail; ++head) {
           const tma::PendEntry& e = S.pend[head % kPendRing];
           publish_item(P, e.op, e.fidx);

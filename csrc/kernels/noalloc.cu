@@ -135,6 +135,7 @@ extern "C" int sar_emulated_allreduce_noalloc(const sar_table* table, void* cons
       P.comm.buf[q] = bufs[q];
     }
     P.ops = d_ops; P.round_begin = d_rb; P.num_rounds = nrb > 0 ? (uint32_t)(nrb - 1) : 0;
+    P.num_ops = (uint32_t)nops; P.one_device = 1;
     P.geom = g; P.rank = r; P.nranks = n; P.participants = sar_table_participants(table);
     P.epoch_base = SAR_VER_STRIDE; P.scale = scale; P.dtype = dtype;
     P.timeout_ns = 10000000000ull;

@@ -19,12 +19,13 @@ enum SarPath { SAR_PATH_SIMT = 0, SAR_PATH_TMA = 1, SAR_PATH_SIMTA = 2 };
 // blocks <= 0 picks the default for the path.  threads is used by the simt
 // path only (<= 0: 512).
 int sar_cuda_launch(const struct SarLaunchParams* p, int path, int blocks, int threads, void* stream);
-// n ranks emulated on the current device by ONE cooperative launch: d_params
-// points to n SarLaunchParams in device memory; rank r is run by blocks
-// [r*blocks_per_rank, (r+1)*blocks_per_rank).  Fails with
+// n ranks emulated on the current device by ONE cooperative launch: params
+// points to n SarLaunchParams in host memory (read during the call), which
+// differ in rank, table, status, trace, delay and the caller's tensors only;
+// rank r is run by blocks [r*blocks_per_rank, (r+1)*blocks_per_rank).  Fails with
 // cudaErrorCooperativeLaunchTooLarge when the blocks cannot all be resident.
-int sar_cuda_launch_emulated(const struct SarLaunchParams* d_params, int n, int dtype, int path, int blocks_per_rank,
-                             int threads, void* stream);
+int sar_cuda_launch_emulated(const struct SarLaunchParams* params, int n, int path, int blocks_per_rank, int threads,
+                             void* stream);
 int sar_cuda_default_blocks(int path);
 // blocks per rank for a buffer of `bytes`: few for small messages (latency bound, and the SMs
 // are left to the compute that overlaps the collective), up to 128 for large ones

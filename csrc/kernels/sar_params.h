@@ -26,6 +26,8 @@ struct SarLaunchParams {
   const SarOp* ops;
   const uint16_t* round_begin;  // num_rounds + 1 entries
   uint32_t num_rounds;
+  uint32_t num_ops;             // round_begin[num_rounds]
+  uint32_t one_device;          // != 0: every rank of the launch runs on this device (fences at device scope suffice)
   SarGeom geom;
   int32_t rank, nranks;
   uint32_t participants;
@@ -57,3 +59,22 @@ struct SarLaunchParams {
   SarMcGroup mc[2];       // multicast views (simt path): all ranks, and e.g. the non-stragglers
 };
 
+
+// Launch parameters of n ranks emulated on one device: what the ranks share once, and per rank what differs.  Passed
+// to the kernel by value (2.7 KB of the 32 KB a launch may carry), so a collective is one launch and no copy.
+// (A copy to device memory ahead of the launch cost 5 us between the two on the stream and 6 us on the host.)
+struct SarEmulRank {
+  const SarOp* ops;
+  const uint16_t* round_begin;
+  uint32_t* status;
+  uint64_t* trace;
+  const void* user_in;
+  void* user_out;
+  uint64_t delay_ns;
+  uint32_t num_rounds, num_ops;
+  uint8_t final_ver[SAR_MAX_CHUNKS];
+};
+struct SarEmulParams {
+  SarLaunchParams common;   // rank 0's parameters
+  SarEmulRank rank[SAR_MAX_RANKS];
+};

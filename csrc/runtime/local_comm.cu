@@ -14,7 +14,7 @@
 #include "symm_alloc.h"
 
 namespace {
-struct DevTable { SarOp* ops = nullptr; uint16_t* round_begin = nullptr; uint32_t num_rounds = 0; };
+struct DevTable { SarOp* ops = nullptr; uint16_t* round_begin = nullptr; uint32_t num_rounds = 0, num_ops = 0; };
 struct Rank {
   int dev = 0;
   cudaStream_t stream = nullptr;
@@ -33,7 +33,6 @@ struct sar_local_comm {
   bool emulate = false;
   std::vector<Rank> ranks;
   uint64_t epoch[SAR_NUM_CHANNELS] = {};   // 64-bit: the low word is the flag epoch, the whole value the gate base
-  SarLaunchParams* d_params = nullptr;   // emulate: n entries on devices[0]
   std::vector<sar::SymmAlloc*> allocs;   // symmetric buffers handed out by sar_local_alloc
 };
 
@@ -95,6 +94,7 @@ static DevTable* upload(Rank& rk, const sar_table* t, int rank, char* err, int e
   if (nops) CK(cudaMemcpy(d.ops, sar_table_ops(t, rank), sizeof(SarOp) * nops, cudaMemcpyHostToDevice));
   if (nrb) CK(cudaMemcpy(d.round_begin, sar_table_round_begin(t, rank), sizeof(uint16_t) * nrb, cudaMemcpyHostToDevice));
   d.num_rounds = nrb > 0 ? (uint32_t)(nrb - 1) : 0;
+  d.num_ops = nops > 0 ? (uint32_t)nops : 0;
   return &(rk.tables[key] = d);
 }
 
@@ -127,10 +127,7 @@ sar_local_comm* sar_local_create(int n, const int* devices, int emulate, char* e
     CK(cudaEventCreate(&rk.ev0));
     CK(cudaEventCreate(&rk.ev1));
   }
-  if (emulate) {
-    CK(cudaSetDevice(devices[0]));
-    CK(cudaMalloc(&c->d_params, sizeof(SarLaunchParams) * n));
-  } else {
+  if (!emulate) {
     for (int a = 0; a < n; ++a) {
       CK(cudaSetDevice(c->ranks[a].dev));
       for (int b = 0; b < n; ++b) {
@@ -162,7 +159,6 @@ void sar_local_destroy(sar_local_comm* c) {
     cudaEventDestroy(rk.ev0); cudaEventDestroy(rk.ev1);
     if (!(c->emulate && r > 0)) cudaStreamDestroy(rk.stream);
   }
-  if (c->d_params) { cudaSetDevice(c->ranks[0].dev); cudaFree(c->d_params); }
   for (sar::SymmAlloc* a : c->allocs) { sar::symm_free(a); delete a; }
   delete c;
 }
@@ -239,7 +235,8 @@ int sar_local_run(sar_local_comm* c, const sar_program* prog, void* const* bufs,
       CK(cudaSetDevice(rk.dev));
       DevTable* dt = upload(rk, t, r, err, errlen);
       if (!dt) return 1;
-      P.ops = dt->ops; P.round_begin = dt->round_begin; P.num_rounds = dt->num_rounds;
+      P.ops = dt->ops; P.round_begin = dt->round_begin; P.num_rounds = dt->num_rounds; P.num_ops = dt->num_ops;
+      P.one_device = c->emulate || n == 1;
       P.geom = g; P.rank = r; P.nranks = n; P.participants = parts;
       P.epoch_base = (uint32_t)c->epoch[ch]; P.gate_base = c->epoch[ch]; P.scale = o->scale; P.dtype = dtype;
       P.timeout_ns = (uint64_t)(timeout_s * 1e9);
@@ -281,9 +278,7 @@ int sar_local_run(sar_local_comm* c, const sar_program* prog, void* const* bufs,
     CK(cudaSetDevice(r0.dev));
     if (o->timed) CK(cudaEventRecord(r0.ev0, r0.stream));
     for (int ph = 0; ph < nph; ++ph) {
-      CK(cudaMemcpyAsync(c->d_params, launches[ph].hp.data(), sizeof(SarLaunchParams) * n, cudaMemcpyHostToDevice, r0.stream));
-      // the copy is from pageable memory: it has completed with respect to the host buffer on return
-      cudaError_t e = (cudaError_t)sar_cuda_launch_emulated(c->d_params, n, dtype, path, launches[ph].blocks, o->threads, r0.stream);
+      cudaError_t e = (cudaError_t)sar_cuda_launch_emulated(launches[ph].hp.data(), n, path, launches[ph].blocks, o->threads, r0.stream);
       if (e != cudaSuccess) {
         if (err) snprintf(err, errlen, "emulated launch (%d ranks x %d blocks): %s", n, launches[ph].blocks, cudaGetErrorString(e));
         return (int)e;
