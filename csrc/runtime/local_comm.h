@@ -40,6 +40,9 @@ sar_local_comm* sar_local_create(int n, const int* devices, int emulate, char* e
 void sar_local_destroy(sar_local_comm* c);
 int sar_local_nranks(const sar_local_comm* c);
 void* sar_local_stream(sar_local_comm* c, int rank);
+// Makes rank's stream wait for what is queued on `stream` (a stream of the rank's device) at this moment.  Returns a
+// cudaError_t.
+int sar_local_wait_stream(sar_local_comm* c, int rank, void* stream);
 // Enqueues the program on every participating rank.  bufs[r] is rank r's buffer
 // (count elements of dtype, 16-byte aligned).  delay_ns may be NULL; a non-zero
 // entry delays that rank on the device before its first phase.  Returns 0 or a

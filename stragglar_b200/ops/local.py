@@ -36,6 +36,7 @@ def cuda_lib():
         L.sar_local_create.argtypes = [C.c_int, C.POINTER(C.c_int), C.c_int, C.c_char_p, C.c_int]
         L.sar_local_destroy.argtypes = [C.c_void_p]
         L.sar_local_stream.restype, L.sar_local_stream.argtypes = C.c_void_p, [C.c_void_p, C.c_int]
+        L.sar_local_wait_stream.restype, L.sar_local_wait_stream.argtypes = C.c_int, [C.c_void_p, C.c_int, C.c_void_p]
         L.sar_local_run.restype = C.c_int
         L.sar_local_run.argtypes = [C.c_void_p, C.c_void_p, C.POINTER(C.c_void_p), C.c_uint64, C.c_int,
                                     C.POINTER(RunOpts), C.POINTER(C.c_uint64), C.c_char_p, C.c_int]
@@ -156,8 +157,9 @@ class LocalComm:
         if len(tensors) != self.n:
             raise ValueError(f"need {self.n} tensors")
         t0 = tensors[0]
+        dtype, numel = t0.dtype, t0.numel()
         for t in tensors:
-            if t.dtype != t0.dtype or t.numel() != t0.numel() or not t.is_contiguous() or not t.is_cuda:
+            if t.dtype != dtype or t.numel() != numel or not t.is_contiguous() or not t.is_cuda:
                 raise ValueError("tensors must be contiguous CUDA tensors of one dtype and size")
         if program._h is None:
             raise ValueError("program was freed")
@@ -166,7 +168,7 @@ class LocalComm:
         uin = None
         udt = 0
         if user_tensors is not None:
-            if len(user_tensors) != self.n or any(u.numel() != t0.numel() or not u.is_contiguous() for u in user_tensors):
+            if len(user_tensors) != self.n or any(u.numel() != numel or not u.is_contiguous() for u in user_tensors):
                 raise ValueError("user_tensors: one contiguous tensor of the same numel per rank")
             uin = (C.c_void_p * self.n)(*[u.data_ptr() for u in user_tensors])
             udt = _dtype_code(user_tensors[0])
@@ -177,14 +179,25 @@ class LocalComm:
         # The ranks run on streams of the communicator: make them wait for what the caller has queued on the
         # current torch stream of every device involved (fills, clones, reference sums), so that the collective
         # neither reads inputs that are not written yet nor overwrites tensors that are still being read.
+        # One event per device and stream of the communicator: emulated ranks share both, and eight event pairs made
+        # through torch were most of a small collective's time on the host.
         import torch
-        for r in range(self.n):
-            dev = tensors[r].device
-            ev = torch.cuda.Event()
-            ev.record(torch.cuda.current_stream(dev))
-            torch.cuda.ExternalStream(cuda_lib().sar_local_stream(self._h, r), device=dev).wait_event(ev)
+        L = cuda_lib()
+        ordered = set()
+        for r, t in enumerate(tensors):
+            dev = t.get_device()
+            key = dev if self.emulate else (dev, r)
+            if key in ordered:
+                continue
+            ordered.add(key)
+            if dev == self.devices[0 if self.emulate else r]:
+                _check(L.sar_local_wait_stream(self._h, r, torch.cuda.current_stream(dev).cuda_stream), "stream order")
+            else:   # a tensor of another device than the rank's
+                ev = torch.cuda.Event()
+                ev.record(torch.cuda.current_stream(dev))
+                torch.cuda.ExternalStream(L.sar_local_stream(self._h, r), device=t.device).wait_event(ev)
         err = C.create_string_buffer(256)
-        rc = cuda_lib().sar_local_run(self._h, program._h, ptrs, t0.numel(), _dtype_code(t0), C.byref(opts), dl, err, 256)
+        rc = L.sar_local_run(self._h, program._h, ptrs, numel, _dtype_code(t0), C.byref(opts), dl, err, 256)
         if rc:
             raise RuntimeError(f"launch failed ({rc}): {err.value.decode()}")
 
