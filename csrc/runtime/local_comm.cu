@@ -6,6 +6,7 @@
 #include <cstring>
 #include <map>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include "../core/host_exec.h"
@@ -34,6 +35,7 @@ struct sar_local_comm {
   bool emulate = false;
   std::vector<Rank> ranks;
   uint64_t epoch[SAR_NUM_CHANNELS] = {};   // 64-bit: the low word is the flag epoch, the whole value the gate base
+  std::map<std::tuple<int, int, int>, int> resident;   // emulate: blocks that fit the device, by (dtype, path, threads)
   std::vector<sar::SymmAlloc*> allocs;   // symmetric buffers handed out by sar_local_alloc
 };
 
@@ -105,6 +107,24 @@ static DevTable* upload(Rank& rk, const sar_table* t, int rank, char* err, int e
   d.num_rounds = nrb > 0 ? (uint32_t)(nrb - 1) : 0;
   d.num_ops = nops > 0 ? (uint32_t)nops : 0;
   return &(rk.tables[key] = d);
+}
+
+// Launch shape of a collective whose ranks share one device: as many blocks per rank as can be resident together,
+// but no more than one per 16 KiB of a rank's buffer (tiles start at 2 KiB: below that the blocks find no work and
+// only lengthen the entry).  Every block is a serial chain of wait, move, announce, so bandwidth comes from their
+// number.  On the simt path 256 threads a block let two chains share an SM where 512 leave it one.
+// 8 ranks, fp32, against 4 blocks per rank: 25 MiB 742 -> 199 us, 256 MiB 7.68 -> 1.61 ms, a staged 25 MiB bucket
+// 2.57 -> 0.45 ms (0.62 ms with a quarter of the blocks staging); 6 ranks, simt, 12 MB 349 -> 70 us (76 us with 512
+// threads a block).
+static int emulated_blocks(sar_local_comm* c, int dtype, int path, int* threads, uint64_t bytes) {
+  if (path == SAR_PATH_SIMT && *threads <= 0) *threads = 256;
+  cudaSetDevice(c->ranks[0].dev);   // occupancy is that of the current device
+  const auto key = std::make_tuple(dtype, path, *threads);
+  auto it = c->resident.find(key);
+  if (it == c->resident.end()) it = c->resident.emplace(key, sar_cuda_max_emulated_blocks(dtype, path, *threads)).first;
+  const uint64_t fit = (uint64_t)(it->second / c->n), want = (bytes + (16u << 10) - 1) / (16u << 10);
+  const uint64_t b = want < 4 ? 4 : want;
+  return (int)(b < fit ? b : (fit < 1 ? 1 : fit));
 }
 
 extern "C" {
@@ -202,7 +222,8 @@ int sar_local_run(sar_local_comm* c, const sar_program* prog, void* const* bufs,
   const uint32_t esize = dtype == SAR_F32 ? 4 : 2;
   const int path = o->path;
   int blocks = o->blocks > 0 ? o->blocks : sar_cuda_pick_blocks(path, count * esize);
-  if (c->emulate && o->blocks <= 0) blocks = 4;   // all ranks share one device
+  int threads = o->threads;
+  if (c->emulate && o->blocks <= 0) blocks = emulated_blocks(c, dtype, path, &threads, count * esize);
   if (n == 1 && o->blocks <= 0 && blocks == 128) blocks = 148;   // a lone rank streams its own memory: one block per SM
   const double timeout_s = o->timeout_s > 0 ? o->timeout_s : 10.0;
   const uint32_t tile_max = o->tile_bytes ? o->tile_bytes : sar_cuda_default_tile_bytes(path);
@@ -274,6 +295,10 @@ int sar_local_run(sar_local_comm* c, const sar_program* prog, void* const* bufs,
       if (o->user_in && o->user_out) {
         P.user_in = o->user_in[r]; P.user_out = o->user_out[r]; P.user_dtype = o->user_dtype;
         sar_table_final_ver(t, r, P.final_ver);
+        // A staged collective moves each byte of a rank in and out on top of the table's traffic (4 S against 3 S for
+        // `stragglar` on 8 ranks), and here both sides run at memory speed: half of the blocks stage
+        // (figures at emulated_blocks).
+        if (c->emulate && o->blocks <= 0 && pblocks >= 2) P.staging_blocks = (uint32_t)pblocks / 2;
       }
       P.delay_ns = 0;
       if (c->emulate && delay_ns && delay_ns[r] && !delayed[r] && (parts >> r & 1)) { P.delay_ns = delay_ns[r]; delayed[r] = true; }
@@ -296,7 +321,7 @@ int sar_local_run(sar_local_comm* c, const sar_program* prog, void* const* bufs,
     CK(cudaSetDevice(r0.dev));
     if (o->timed) CK(cudaEventRecord(r0.ev0, r0.stream));
     for (int ph = 0; ph < nph; ++ph) {
-      cudaError_t e = (cudaError_t)sar_cuda_launch_emulated(launches[ph].hp.data(), n, path, launches[ph].blocks, o->threads, r0.stream);
+      cudaError_t e = (cudaError_t)sar_cuda_launch_emulated(launches[ph].hp.data(), n, path, launches[ph].blocks, threads, r0.stream);
       if (e != cudaSuccess) {
         if (err) snprintf(err, errlen, "emulated launch (%d ranks x %d blocks): %s", n, launches[ph].blocks, cudaGetErrorString(e));
         return (int)e;

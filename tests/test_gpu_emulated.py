@@ -279,3 +279,26 @@ def test_staged_mode_reads_and_writes_the_callers_tensors(alg, n, wire, user, pa
         for u in users:
             torch.testing.assert_close(u.double(), want, **tol)
     comm.close()
+
+
+@pytest.mark.parametrize("path", PATHS)
+@pytest.mark.parametrize("n,count", [(8, 1), (8, 8 * 4096 + 3), (6, 16 * 4096 - 1), (16, 300_007), (2, 2_000_003)])
+@pytest.mark.parametrize("staged", [False, True])
+def test_default_launch_shape(n, count, staged, path):
+    """The launch shape chosen for emulated ranks (from one item of work to more than the device holds at once)
+    against two blocks per rank: the split of the work never touches the order of a sum, so the bits are equal."""
+    from stragglar_b200 import ops
+    comm = ops.LocalComm(n, emulate=True)
+    prog = sc.compile_program("stragglar", n)
+    outs = []
+    for kw in ({}, {"blocks": 2}):
+        xs = _inputs(n, count, torch.float32)
+        arena = [torch.zeros_like(x) for x in xs] if staged else xs
+        comm.run(prog, arena, path=path, scale=1.0 / n, timeout_s=5.0, user_tensors=xs if staged else None, **kw)
+        comm.sync()
+        outs.append(xs)
+    want = torch.stack([x.double() for x in _inputs(n, count, torch.float32)]).mean(0)
+    for a, b in zip(*outs):
+        assert torch.equal(a, b)
+        torch.testing.assert_close(a.double(), want, **TOL[torch.float32])
+    comm.close()
