@@ -282,9 +282,11 @@ int sar_cuda_launch(const SarLaunchParams* p, int path, int blocks, int threads,
   return with_dtype(p->dtype, [&](auto tag) -> int {
     using T = decltype(tag);
     if (path == SAR_PATH_TMA) {
-      int e = allow_smem(sar_exec_tma_kernel<T>, sizeof(tma::Shared));
+      // always the whole ring: ranks on devices of their own have an SM to themselves
+      const uint32_t smem = tma::smem_bytes(table_ops(*p), tma::kStages);
+      int e = allow_smem(sar_exec_tma_kernel<T>, smem);
       if (e) return e;
-      sar_exec_tma_kernel<T><<<blocks, tma::kThreads, sizeof(tma::Shared), st>>>(*p);
+      sar_exec_tma_kernel<T><<<blocks, tma::kThreads, smem, st>>>(*p);
     } else if (path == SAR_PATH_SIMTA) {
       sar_exec_simta_kernel<T><<<blocks, simta::kThreads, 0, st>>>(*p);
     } else {
@@ -296,13 +298,18 @@ int sar_cuda_launch(const SarLaunchParams* p, int path, int blocks, int threads,
 }
 
 int sar_cuda_max_emulated_blocks(int dtype, int path, int threads) {
+  return sar_cuda_emulated_fit(dtype, path, threads, 0, SAR_MAX_OPS);
+}
+
+int sar_cuda_emulated_fit(int dtype, int path, int threads, int stages, int num_ops) {
   int dev = 0, sms = 0, per_sm = 0;
   if (cudaGetDevice(&dev) || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) return 0;
   with_dtype(dtype, [&](auto tag) -> int {
     using T = decltype(tag);
     if (path == SAR_PATH_TMA) {
-      allow_smem(sar_emul_tma_kernel<T>, sizeof(tma::Shared));
-      return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sar_emul_tma_kernel<T>, tma::kThreads, sizeof(tma::Shared));
+      const uint32_t smem = tma::smem_bytes((uint32_t)num_ops, tma::stages_in_use((uint32_t)stages));
+      allow_smem(sar_emul_tma_kernel<T>, smem);
+      return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sar_emul_tma_kernel<T>, tma::kThreads, smem);
     }
     if (path == SAR_PATH_SIMTA)
       return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sar_emul_simta_kernel<T>, simta::kThreads, 0);
@@ -330,10 +337,13 @@ int sar_cuda_launch_emulated(const SarLaunchParams* params, int n, int path, int
     using T = decltype(tag);
     void* args[] = {(void*)&E, (void*)&blocks_per_rank};
     if (path == SAR_PATH_TMA) {
-      int e = allow_smem(sar_emul_tma_kernel<T>, sizeof(tma::Shared));
+      uint32_t nops = 0;
+      for (int r = 0; r < n; ++r) nops = table_ops(params[r]) > nops ? table_ops(params[r]) : nops;
+      const uint32_t smem = tma::smem_bytes(nops, tma::stages_in_use(E.common.stages));
+      int e = allow_smem(sar_emul_tma_kernel<T>, smem);
       if (e) return e;
       return (int)cudaLaunchCooperativeKernel((void*)sar_emul_tma_kernel<T>, dim3(n * blocks_per_rank), dim3(tma::kThreads),
-                                              args, sizeof(tma::Shared), st);
+                                              args, smem, st);
     }
     if (path == SAR_PATH_SIMTA)
       return (int)cudaLaunchCooperativeKernel((void*)sar_emul_simta_kernel<T>, dim3(n * blocks_per_rank), dim3(simta::kThreads), args, 0, st);

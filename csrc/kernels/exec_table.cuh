@@ -241,8 +241,8 @@ struct OpGeom {
 };
 struct RoundGeom { uint32_t op_begin, m, max_tiles, pad; };
 struct TableGeom {
-  SarOp ops[SAR_MAX_OPS];               // the rank's table itself: read for every piece by every role of the block
-  OpGeom op[SAR_MAX_OPS];
+  SarOp* ops;                           // the rank's table itself: read for every piece by every role of the block
+  OpGeom* op;                           // (both in shared memory, room for num_ops entries)
   uint16_t round_begin[SAR_MAX_ROUNDS + 1];
   RoundGeom round[2][SAR_MAX_ROUNDS];   // per lane
   SarOp stage_op[2];                    // pseudo ops of staged mode: [0] SAR_STAGE_IN, [1] SAR_STAGE_OUT
@@ -265,6 +265,8 @@ __device__ __forceinline__ uint32_t staging_blocks(const SarLaunchParams& P, uin
   return nblocks >= 8 ? nblocks / 4 : 1u;
 }
 
+__host__ __device__ __forceinline__ uint32_t table_ops(const SarLaunchParams& P) { return P.num_ops < SAR_MAX_OPS ? P.num_ops : SAR_MAX_OPS; }
+
 // All threads of the block; ends with a block barrier.
 //
 // Bound by latency, on the path of every collective: the table is fetched with one round of coalesced loads (ops and
@@ -273,11 +275,12 @@ __device__ __forceinline__ uint32_t staging_blocks(const SarLaunchParams& P, uin
 // another one, because the acquiring fences of the waits empty L1.
 // Eight ranks on one device, 4 KiB: 38 -> 19 us in the kernel (rsag, bulk-copy path), 34 -> 15 us (simt); of that the
 // fences at device scope and the flag polls kept in registers (wait_item_ready) are about half.
-__device__ void resolve_table(const SarLaunchParams& P, TableGeom& G, uint32_t nblocks) {
+__device__ void resolve_table(const SarLaunchParams& P, TableGeom& G, uint32_t nblocks, SarOp* ops_mem, OpGeom* op_mem) {
   const uint32_t nrounds = P.num_rounds < SAR_MAX_ROUNDS ? P.num_rounds : SAR_MAX_ROUNDS;
-  const uint32_t nops = nrounds ? (P.num_ops < SAR_MAX_OPS ? P.num_ops : SAR_MAX_OPS) : 0;
+  const uint32_t nops = nrounds ? table_ops(P) : 0;
   for (uint32_t i = threadIdx.x; i < nops * (sizeof(SarOp) / 4); i += blockDim.x)
-    reinterpret_cast<uint32_t*>(G.ops)[i] = reinterpret_cast<const uint32_t*>(P.ops)[i];
+    reinterpret_cast<uint32_t*>(ops_mem)[i] = reinterpret_cast<const uint32_t*>(P.ops)[i];
+  if (threadIdx.x == 0) { G.ops = ops_mem; G.op = op_mem; }
   if (nrounds)
     for (uint32_t r = threadIdx.x; r <= nrounds; r += blockDim.x) G.round_begin[r] = P.round_begin[r];
   __syncthreads();
@@ -892,10 +895,12 @@ __device__ void leave_collective(const SarLaunchParams& P, const WaitCtx& w, uin
 template <typename T>
 __device__ void run_rank_simt(const SarLaunchParams& P, uint32_t block, uint32_t nblocks) {
   __shared__ TableGeom G;
+  __shared__ SarOp s_ops[SAR_MAX_OPS];
+  __shared__ OpGeom s_op[SAR_MAX_OPS];
   __shared__ Item s_item;
   __shared__ int s_state;   // 1: item ready, 0: table exhausted, -1: a wait failed
   WaitCtx w = enter_collective(P, block);
-  resolve_table(P, G, nblocks);
+  resolve_table(P, G, nblocks, s_ops, s_op);
   ItemWalker walk;
   uint32_t arrived = 1u << P.rank, gate_passed = 0;
   if (threadIdx.x == 0) {
@@ -960,8 +965,13 @@ struct StageDesc {
 };
 struct PendEntry { const SarOp* op; uint32_t fidx; uint32_t seq; };
 
+// Dynamic shared memory of a block: this structure, the op table (ops_offset), and the ring of `stages` stages
+// (ring_offset).  A launch that asks for fewer than kStages stages may allocate just those.
+// Ranks on one device: a block is a serial chain (wait, load, add, store, announce) at some 27 GB/s, whatever its ring
+// holds, so two blocks with three stages each share an SM instead of one with six.  8 ranks, fp32: 25 MiB 206 -> 141 us,
+// 256 MiB 1634 -> 1137 us, a staged 25 MiB bucket 464 -> 323 us.  Three blocks with two stages: 195 us at 25 MiB (a
+// stage is handed back one piece late, which leaves a ring of two with nothing in flight).
 struct Shared {
-  alignas(128) unsigned char ring[kStages][kStageBytes];
   alignas(8) uint64_t full[kStages];
   alignas(8) uint64_t empty[kStages];
   StageDesc desc[kStages];
@@ -975,6 +985,14 @@ struct Shared {
   int abort_seen;
   uint32_t issued;      // pieces the producer has issued (written when it stops)
 };
+
+// ring stages in use: fewer stages keep fewer bytes in flight per block
+__host__ __device__ __forceinline__ uint32_t stages_in_use(uint32_t asked) { return (asked >= 2 && asked < (uint32_t)kStages) ? asked : (uint32_t)kStages; }
+__host__ __device__ __forceinline__ uint32_t ops_offset() { return (uint32_t)((sizeof(Shared) + 15) / 16 * 16); }
+__host__ __device__ __forceinline__ uint32_t ring_offset(uint32_t nops) {
+  return (uint32_t)((ops_offset() + nops * (sizeof(OpGeom) + sizeof(SarOp)) + 127) / 128 * 128);
+}
+__host__ __device__ __forceinline__ uint32_t smem_bytes(uint32_t nops, uint32_t stages) { return ring_offset(nops) + stages * (uint32_t)kStageBytes; }
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void mbar_init(uint64_t* b, uint32_t count) {
@@ -1058,8 +1076,9 @@ __device__ void run_rank_tma(const SarLaunchParams& P, uint32_t block, uint32_t 
   constexpr int N = Vec<T>::N;
   const uint32_t tid = threadIdx.x;
   const uint32_t warp = tid >> 5, lane = tid & 31;
-  // ring stages in use: fewer stages keep fewer bytes in flight per block
-  const uint32_t nst = (P.stages >= 2 && P.stages < (uint32_t)kStages) ? P.stages : (uint32_t)kStages;
+  const uint32_t nst = stages_in_use(P.stages);
+  unsigned char* const ring = reinterpret_cast<unsigned char*>(&S) + ring_offset(table_ops(P));
+  OpGeom* const op_mem = reinterpret_cast<OpGeom*>(reinterpret_cast<unsigned char*>(&S) + ops_offset());
   WaitCtx w = enter_collective(P, block);
   if (tid == 0) {
     for (int s = 0; s < kStages; ++s) { mbar_init(&S.full[s], 1); mbar_init(&S.empty[s], 1); }
@@ -1068,7 +1087,7 @@ __device__ void run_rank_tma(const SarLaunchParams& P, uint32_t block, uint32_t 
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     fence_proxy_async();
   }
-  resolve_table(P, S.geom, nblocks);   // ends with a block barrier
+  resolve_table(P, S.geom, nblocks, reinterpret_cast<SarOp*>(op_mem + table_ops(P)), op_mem);   // ends with a block barrier
 
   if (warp == 0) {
     // ---------------------------------------------------------------- producer
@@ -1126,7 +1145,7 @@ __device__ void run_rank_tma(const SarLaunchParams& P, uint32_t block, uint32_t 
             d.tail_elem0 = it.elem0 + body;
             if (pe) {
               mbar_arrive_expect_tx(&S.full[s], d.bytes);
-              bulk_load(&S.ring[s][0], src + d.byte_off, d.bytes, &S.full[s]);
+              bulk_load(ring + s * kStageBytes, src + d.byte_off, d.bytes, &S.full[s]);
             } else {
               mbar_arrive(&S.full[s]);
             }
@@ -1156,9 +1175,9 @@ __device__ void run_rank_tma(const SarLaunchParams& P, uint32_t block, uint32_t 
           if (bytes) {
             mbar_arrive_expect_tx(&S.full[s], bytes * nsrc_total);
             for (uint32_t q = 0; q < npeer; ++q)
-              bulk_load(&S.ring[s][q * slot_bytes], (const char*)P.comm.buf[op->src[q]] + d.byte_off, bytes, &S.full[s]);
+              bulk_load(ring + s * kStageBytes + q * slot_bytes, (const char*)P.comm.buf[op->src[q]] + d.byte_off, bytes, &S.full[s]);
             if (local)
-              bulk_load(&S.ring[s][npeer * slot_bytes], (const char*)P.comm.buf[P.rank] + d.byte_off, bytes, &S.full[s]);
+              bulk_load(ring + s * kStageBytes + npeer * slot_bytes, (const char*)P.comm.buf[P.rank] + d.byte_off, bytes, &S.full[s]);
           } else {
             mbar_arrive(&S.full[s]);   // an item that is only a sub-vector tail
           }
@@ -1206,7 +1225,7 @@ __device__ void run_rank_tma(const SarLaunchParams& P, uint32_t block, uint32_t 
       const StageDesc d = S.desc[s];
       if (d.op == nullptr) break;
       const SarOp* op = d.op;
-      unsigned char* stage = S.ring[s];
+      unsigned char* stage = ring + s * kStageBytes;
       if (op->kind >= SAR_STAGE_IN) {
         if (d.item_elems) {
           Item sit{};
@@ -1394,6 +1413,8 @@ constexpr int kPendRing = 16;
 
 struct Shared {
   TableGeom geom;
+  SarOp ops[SAR_MAX_OPS];
+  OpGeom op[SAR_MAX_OPS];
   Item slot[kSlots];
   int state[kSlots];          // 1: item ready, 0: table exhausted, -1: a wait failed
   int decision;               // the state the workers act on (written by worker thread 0)
@@ -1423,7 +1444,7 @@ __device__ void run_rank_simta(const SarLaunchParams& P, uint32_t block, uint32_
     S.pend_tail = 0; S.pend_head = 0; S.workers_done = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  resolve_table(P, S.geom, nblocks);   // ends with a block barrier
+  resolve_table(P, S.geom, nblocks, S.ops, S.op);   // ends with a block barrier
 
   if (warp < (uint32_t)kWorkerWarps) {
     // ----------------------------------------------------------------- workers

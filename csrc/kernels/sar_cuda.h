@@ -32,6 +32,8 @@ int sar_cuda_default_blocks(int path);
 int sar_cuda_pick_blocks(int path, uint64_t bytes);
 uint32_t sar_cuda_default_tile_bytes(int path);
 int sar_cuda_max_emulated_blocks(int dtype, int path, int threads);   // resident blocks on the current device
+// the same for a launch with `stages` ring stages (0: all; bulk-copy path) and tables of at most num_ops ops
+int sar_cuda_emulated_fit(int dtype, int path, int threads, int stages, int num_ops);
 
 // Barrier across ranks on control channel `channel`: announces `epoch` and
 // waits (bounded) until every rank in `participants` has announced it.

@@ -2,6 +2,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdio>
 #include <cstring>
 #include <map>
@@ -35,7 +36,8 @@ struct sar_local_comm {
   bool emulate = false;
   std::vector<Rank> ranks;
   uint64_t epoch[SAR_NUM_CHANNELS] = {};   // 64-bit: the low word is the flag epoch, the whole value the gate base
-  std::map<std::tuple<int, int, int>, int> resident;   // emulate: blocks that fit the device, by (dtype, path, threads)
+  // emulate: blocks that fit the device, by (dtype, path, threads, ring stages, ops in the table)
+  std::map<std::tuple<int, int, int, int, int>, int> resident;
   std::vector<sar::SymmAlloc*> allocs;   // symmetric buffers handed out by sar_local_alloc
 };
 
@@ -114,14 +116,19 @@ static DevTable* upload(Rank& rk, const sar_table* t, int rank, char* err, int e
 // only lengthen the entry).  Every block is a serial chain of wait, move, announce, so bandwidth comes from their
 // number.  On the simt path 256 threads a block let two chains share an SM where 512 leave it one.
 // 8 ranks, fp32, against 4 blocks per rank: 25 MiB 742 -> 199 us, 256 MiB 7.68 -> 1.61 ms, a staged 25 MiB bucket
-// 2.57 -> 0.45 ms (0.62 ms with a quarter of the blocks staging); 6 ranks, simt, 12 MB 349 -> 70 us (76 us with 512
+// 2.57 -> 0.45 ms (0.62 ms with a quarter of the blocks staging; these with one bulk-copy block per SM, two since then:
+// see tma::Shared); 6 ranks, simt, 12 MB 349 -> 70 us (76 us with 512
 // threads a block).
-static int emulated_blocks(sar_local_comm* c, int dtype, int path, int* threads, uint64_t bytes) {
+static int emulated_blocks(sar_local_comm* c, const sar_program* prog, int dtype, int path, int* threads, int stages, uint64_t bytes) {
   if (path == SAR_PATH_SIMT && *threads <= 0) *threads = 256;
   cudaSetDevice(c->ranks[0].dev);   // occupancy is that of the current device
-  const auto key = std::make_tuple(dtype, path, *threads);
+  int nops = 0;
+  if (path == SAR_PATH_TMA)
+    for (int ph = 0; ph < sar_program_num_phases(prog); ++ph)
+      for (int r = 0; r < c->n; ++r) nops = std::max(nops, sar_table_num_ops(sar_program_phase(prog, ph), r));
+  const auto key = std::make_tuple(dtype, path, *threads, stages, nops);
   auto it = c->resident.find(key);
-  if (it == c->resident.end()) it = c->resident.emplace(key, sar_cuda_max_emulated_blocks(dtype, path, *threads)).first;
+  if (it == c->resident.end()) it = c->resident.emplace(key, sar_cuda_emulated_fit(dtype, path, *threads, stages, nops)).first;
   const uint64_t fit = (uint64_t)(it->second / c->n), want = (bytes + (16u << 10) - 1) / (16u << 10);
   const uint64_t b = want < 4 ? 4 : want;
   return (int)(b < fit ? b : (fit < 1 ? 1 : fit));
@@ -222,8 +229,11 @@ int sar_local_run(sar_local_comm* c, const sar_program* prog, void* const* bufs,
   const uint32_t esize = dtype == SAR_F32 ? 4 : 2;
   const int path = o->path;
   int blocks = o->blocks > 0 ? o->blocks : sar_cuda_pick_blocks(path, count * esize);
-  int threads = o->threads;
-  if (c->emulate && o->blocks <= 0) blocks = emulated_blocks(c, dtype, path, &threads, count * esize);
+  int threads = o->threads, stages = o->stages;
+  if (c->emulate && o->blocks <= 0) {
+    if (path == SAR_PATH_TMA && stages <= 0) stages = 3;   // two blocks per SM (see emulated_blocks)
+    blocks = emulated_blocks(c, prog, dtype, path, &threads, stages, count * esize);
+  }
   if (n == 1 && o->blocks <= 0 && blocks == 128) blocks = 148;   // a lone rank streams its own memory: one block per SM
   const double timeout_s = o->timeout_s > 0 ? o->timeout_s : 10.0;
   const uint32_t tile_max = o->tile_bytes ? o->tile_bytes : sar_cuda_default_tile_bytes(path);
@@ -282,7 +292,7 @@ int sar_local_run(sar_local_comm* c, const sar_program* prog, void* const* bufs,
       P.status = rk.status; P.trace = rk.trace; P.trace_rounds = o->trace_rounds ? 1u : 0u;
       P.gate_rounds = gated ? 1u : 0u;
       P.gate_slack = sar::gate_slack(g.tiles_per_chunk);
-      P.stages = o->stages > 0 ? (uint32_t)o->stages : (uint32_t)sar_table_stages_hint(t);
+      P.stages = stages > 0 ? (uint32_t)stages : (uint32_t)sar_table_stages_hint(t);
       P.store_window = o->store_window > 0 ? (uint32_t)o->store_window : 0u;
       P.lane1_eighths = (uint32_t)sar_table_lane1_eighths(t);
       if (mc_alloc) {
