@@ -1062,6 +1062,68 @@ __device__ __forceinline__ uint32_t pow2_ceil(uint32_t x) {
 }
 }  // namespace tma
 
+// Converts `elems` (a multiple of 8) elements in shared memory with NT threads.  Bound by latency: four elements a
+// thread and turn (16 bytes on the 4-byte side, 8 on the 2-byte side, consecutive threads on consecutive words, so
+// without bank conflicts) and four independent turns at a time.  One type pair is chosen per piece, not per element.
+// 8 ranks, 25 MiB fp32 buckets, bf16 wire: 487 -> 421 us (eight elements a turn at a stride of 32 bytes before), and
+// 270 us with two blocks per SM.
+template <int SDT, int DDT> __device__ __forceinline__ uint4 convert4(uint4 v) {
+  float f[4];
+  if constexpr (SDT == SAR_F32) {
+    f[0] = __uint_as_float(v.x); f[1] = __uint_as_float(v.y); f[2] = __uint_as_float(v.z); f[3] = __uint_as_float(v.w);
+  } else if constexpr (SDT == SAR_BF16) {
+    f[0] = __uint_as_float(v.x << 16); f[1] = __uint_as_float(v.x & 0xffff0000u);
+    f[2] = __uint_as_float(v.y << 16); f[3] = __uint_as_float(v.y & 0xffff0000u);
+  } else {
+    const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&v.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&v.y));
+    f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y;
+  }
+  uint4 o = make_uint4(0, 0, 0, 0);
+  if constexpr (DDT == SAR_F32) {
+    o = make_uint4(__float_as_uint(f[0]), __float_as_uint(f[1]), __float_as_uint(f[2]), __float_as_uint(f[3]));
+  } else if constexpr (DDT == SAR_BF16) {
+    const __nv_bfloat162 a = __floats2bfloat162_rn(f[0], f[1]), b = __floats2bfloat162_rn(f[2], f[3]);
+    o.x = *reinterpret_cast<const uint32_t*>(&a); o.y = *reinterpret_cast<const uint32_t*>(&b);
+  } else {
+    const __half2 a = __floats2half2_rn(f[0], f[1]), b = __floats2half2_rn(f[2], f[3]);
+    o.x = *reinterpret_cast<const uint32_t*>(&a); o.y = *reinterpret_cast<const uint32_t*>(&b);
+  }
+  return o;
+}
+template <int NT, int SDT, int DDT>
+__device__ __forceinline__ void convert_pair(unsigned char* dst, const unsigned char* src, uint32_t elems, uint32_t tid) {
+  const uint32_t n4 = elems / 4;
+  auto load = [&](uint32_t g) -> uint4 {
+    if constexpr (SDT == SAR_F32) return reinterpret_cast<const uint4*>(src)[g];
+    const uint2 t = reinterpret_cast<const uint2*>(src)[g];
+    return make_uint4(t.x, t.y, 0, 0);
+  };
+  auto store = [&](uint32_t g, uint4 v) {
+    if constexpr (DDT == SAR_F32) reinterpret_cast<uint4*>(dst)[g] = v;
+    else reinterpret_cast<uint2*>(dst)[g] = make_uint2(v.x, v.y);
+  };
+  uint32_t g = tid;
+  for (; g + 3 * NT < n4; g += 4 * NT) {
+    uint4 v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) v[u] = load(g + u * NT);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) store(g + u * NT, convert4<SDT, DDT>(v[u]));
+  }
+  for (; g < n4; g += NT) store(g, convert4<SDT, DDT>(load(g)));
+}
+template <int NT>
+__device__ void convert_piece(unsigned char* dst, int ddt, const unsigned char* src, int sdt, uint32_t elems, uint32_t tid) {
+  if (sdt == SAR_F32) {
+    if (ddt == SAR_BF16) convert_pair<NT, SAR_F32, SAR_BF16>(dst, src, elems, tid);
+    else convert_pair<NT, SAR_F32, SAR_F16>(dst, src, elems, tid);
+  } else if (sdt == SAR_BF16) {
+    convert_pair<NT, SAR_BF16, SAR_F32>(dst, src, elems, tid);
+  } else {
+    convert_pair<NT, SAR_F16, SAR_F32>(dst, src, elems, tid);
+  }
+}
+
 // Roles of a block (192 threads):
 //   warp 0, one thread   producer: walks the items, waits for their operands
 //                        (flags in peer memory), streams the tiles into the ring;
@@ -1232,26 +1294,10 @@ __device__ void run_rank_tma(const SarLaunchParams& P, uint32_t block, uint32_t 
           sit.op = op; sit.elem0 = d.item_elem0; sit.nelem = d.item_elems;
           stage_tile<T>(P, sit, ctid, CT);
         } else if (d.bytes != d.dst_bytes) {
-          // convert the piece from the first half of the stage into the second, eight elements per thread and turn
+          // convert the piece from the first half of the stage into the second
           const bool in = op->kind == SAR_STAGE_IN;
           const int sdt = in ? P.user_dtype : P.dtype, ddt = in ? P.dtype : P.user_dtype;
-          unsigned char* out = stage + kStageBytes / 2;
-          for (uint32_t g = ctid; g < d.piece_elems / 8; g += CT) {
-            float f[8];
-            if (sdt == SAR_F32) {
-              const float4 a = *reinterpret_cast<const float4*>(stage + (size_t)g * 32), b = *reinterpret_cast<const float4*>(stage + (size_t)g * 32 + 16);
-              f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
-            } else {
-              const uint4 v = *reinterpret_cast<const uint4*>(stage + (size_t)g * 16);
-              if (sdt == SAR_BF16) Vec<__nv_bfloat16>::unpack(v, f); else Vec<__half>::unpack(v, f);
-            }
-            if (ddt == SAR_F32) {
-              *reinterpret_cast<float4*>(out + (size_t)g * 32) = make_float4(f[0], f[1], f[2], f[3]);
-              *reinterpret_cast<float4*>(out + (size_t)g * 32 + 16) = make_float4(f[4], f[5], f[6], f[7]);
-            } else {
-              *reinterpret_cast<uint4*>(out + (size_t)g * 16) = ddt == SAR_BF16 ? Vec<__nv_bfloat16>::pack(f) : Vec<__half>::pack(f);
-            }
-          }
+          convert_piece<CT>(stage + kStageBytes / 2, ddt, stage, sdt, d.piece_elems, ctid);
           fence_proxy_async_smem();
         }
       } else if (op->kind != SAR_COPY && op->kind != SAR_PUSH && d.bytes) {
