@@ -115,10 +115,8 @@ static DevTable* upload(Rank& rk, const sar_table* t, int rank, char* err, int e
 // but no more than one per 16 KiB of a rank's buffer (tiles start at 2 KiB: below that the blocks find no work and
 // only lengthen the entry).  Every block is a serial chain of wait, move, announce, so bandwidth comes from their
 // number.  On the simt path 256 threads a block let two chains share an SM where 512 leave it one.
-// 8 ranks, fp32, against 4 blocks per rank: 25 MiB 742 -> 199 us, 256 MiB 7.68 -> 1.61 ms, a staged 25 MiB bucket
-// 2.57 -> 0.45 ms (0.62 ms with a quarter of the blocks staging; these with one bulk-copy block per SM, two since then:
-// see tma::Shared); 6 ranks, simt, 12 MB 349 -> 70 us (76 us with 512
-// threads a block).
+// 8 ranks, fp32, against 4 blocks per rank: 25 MiB 742 -> 199 us, 256 MiB 7.68 -> 1.61 ms (one bulk-copy block per SM;
+// two since then, see tma::Shared); 6 ranks, simt, 12 MB 349 -> 70 us (76 us with 512 threads a block).
 static int emulated_blocks(sar_local_comm* c, const sar_program* prog, int dtype, int path, int* threads, int stages, uint64_t bytes) {
   if (path == SAR_PATH_SIMT && *threads <= 0) *threads = 256;
   cudaSetDevice(c->ranks[0].dev);   // occupancy is that of the current device
@@ -305,10 +303,7 @@ int sar_local_run(sar_local_comm* c, const sar_program* prog, void* const* bufs,
       if (o->user_in && o->user_out) {
         P.user_in = o->user_in[r]; P.user_out = o->user_out[r]; P.user_dtype = o->user_dtype;
         sar_table_final_ver(t, r, P.final_ver);
-        // A staged collective moves each byte of a rank in and out on top of the table's traffic (4 S against 3 S for
-        // `stragglar` on 8 ranks), and here both sides run at memory speed: half of the blocks stage
-        // (figures at emulated_blocks).
-        if (c->emulate && o->blocks <= 0 && pblocks >= 2) P.staging_blocks = (uint32_t)pblocks / 2;
+        if (c->emulate && o->blocks <= 0) P.staging_blocks = SAR_STAGE_EVERYWHERE;
       }
       P.delay_ns = 0;
       if (c->emulate && delay_ns && delay_ns[r] && !delayed[r] && (parts >> r & 1)) { P.delay_ns = delay_ns[r]; delayed[r] = true; }
