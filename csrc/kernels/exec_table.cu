@@ -22,7 +22,7 @@ __global__ void __launch_bounds__(tma::kThreads, 1) sar_exec_tma_kernel(const __
 template <typename T>
 __global__ void __launch_bounds__(simta::kThreads, 1) sar_exec_simta_kernel(const __grid_constant__ SarLaunchParams P) {
   __shared__ simta::Shared S;
-  run_rank_simta<T>(P, blockIdx.x, gridDim.x, S);
+  run_rank_simta<T, simta::kThreads>(P, blockIdx.x, gridDim.x, S);
 }
 
 // All ranks of a collective in one launch on one device (tests, profiling).
@@ -54,12 +54,12 @@ __global__ void __launch_bounds__(512, 1) sar_emul_simt_kernel(const __grid_cons
 }
 
 template <typename T>
-__global__ void __launch_bounds__(simta::kThreads, 1) sar_emul_simta_kernel(const __grid_constant__ SarEmulParams E, int blocks_per_rank) {
+__global__ void __launch_bounds__(simta::kThreadsShared, 2) sar_emul_simta_kernel(const __grid_constant__ SarEmulParams E, int blocks_per_rank) {
   __shared__ SarLaunchParams P;
   __shared__ simta::Shared S;
   load_rank_params(E, blockIdx.x / blocks_per_rank, P);
   if (!(P.participants >> P.rank & 1)) return;
-  run_rank_simta<T>(P, blockIdx.x % blocks_per_rank, blocks_per_rank, S);
+  run_rank_simta<T, simta::kThreadsShared>(P, blockIdx.x % blocks_per_rank, blocks_per_rank, S);
 }
 
 template <typename T>
@@ -312,7 +312,7 @@ int sar_cuda_emulated_fit(int dtype, int path, int threads, int stages, int num_
       return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sar_emul_tma_kernel<T>, tma::kThreads, smem);
     }
     if (path == SAR_PATH_SIMTA)
-      return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sar_emul_simta_kernel<T>, simta::kThreads, 0);
+      return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sar_emul_simta_kernel<T>, simta::kThreadsShared, 0);
     return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sar_emul_simt_kernel<T>, threads <= 0 ? 512 : threads, 0);
   });
   return sms * per_sm;
@@ -346,7 +346,7 @@ int sar_cuda_launch_emulated(const SarLaunchParams* params, int n, int path, int
                                               args, smem, st);
     }
     if (path == SAR_PATH_SIMTA)
-      return (int)cudaLaunchCooperativeKernel((void*)sar_emul_simta_kernel<T>, dim3(n * blocks_per_rank), dim3(simta::kThreads), args, 0, st);
+      return (int)cudaLaunchCooperativeKernel((void*)sar_emul_simta_kernel<T>, dim3(n * blocks_per_rank), dim3(simta::kThreadsShared), args, 0, st);
     if (threads <= 0) threads = 512;
     return (int)cudaLaunchCooperativeKernel((void*)sar_emul_simt_kernel<T>, dim3(n * blocks_per_rank), dim3(threads), args, 0, st);
   });

@@ -1479,8 +1479,7 @@ __device__ void run_rank_tma(const SarLaunchParams& P, uint32_t block, uint32_t 
 // reductions over, and pushes to, a whole multicast group go through the switch.
 namespace simta {
 constexpr int kThreads = 512;
-constexpr int kWorkerWarps = 14;
-constexpr int kWorkers = 32 * kWorkerWarps;
+constexpr int kThreadsShared = 256;   // ranks on one device: two blocks per SM (see run_rank_simta)
 constexpr int kSlots = 2;
 constexpr int kPendRing = 16;
 
@@ -1498,12 +1497,16 @@ struct Shared {
   uint32_t pend_head;         // written by the signal thread
   uint32_t workers_done;
 };
-__device__ __forceinline__ void worker_bar() { asm volatile("bar.sync 1, %0;" ::"n"(kWorkers) : "memory"); }
+template <int WORKERS> __device__ __forceinline__ void worker_bar() { asm volatile("bar.sync 1, %0;" ::"n"(WORKERS) : "memory"); }
 }  // namespace simta
 
-template <typename T>
+// THREADS per block: all but the last two warps are workers.  A block moves one tile at a time; with 256 threads two
+// of them fit an SM (125 registers a thread) and one copies while the other turns over.  8 ranks on one device, rhd,
+// 64 MiB fp16: 504 us with one 512-thread block per SM, 443 us with two of 256 threads, 424 us with tiles of 256 KiB.
+template <typename T, int THREADS>
 __device__ void run_rank_simta(const SarLaunchParams& P, uint32_t block, uint32_t nblocks, simta::Shared& S) {
   using namespace simta;
+  constexpr int kWorkerWarps = THREADS / 32 - 2, kWorkers = 32 * kWorkerWarps;
   using tma::ld_acquire_cta;
   using tma::mbar_arrive;
   using tma::mbar_init;
@@ -1530,11 +1533,11 @@ __device__ void run_rank_simta(const SarLaunchParams& P, uint32_t block, uint32_
         const bool ok = mbar_wait(&S.full[s], (seq / kSlots) & 1, w);
         *(volatile int*)&S.decision = ok ? *(volatile int*)&S.state[s] : -1;
       }
-      worker_bar();
+      worker_bar<kWorkers>();
       if (*(volatile int*)&S.decision != 1) break;
       const Item it = S.slot[s];
       simt_tile<T, 4>(P, it, tid, kWorkers);
-      worker_bar();                    // every store of the tile is issued; every worker has read the slot and the decision
+      worker_bar<kWorkers>();                    // every store of the tile is issued; every worker has read the slot and the decision
       if (tid == 0) {
         // hand the item to the signal thread (bounded wait if its ring is full), free the slot
         while (pend_tail - ld_acquire_cta(&S.pend_head) >= (uint32_t)kPendRing) {
