@@ -53,13 +53,13 @@ __global__ void __launch_bounds__(512, 1) sar_emul_simt_kernel(const __grid_cons
   run_rank_simt<T>(P, blockIdx.x % blocks_per_rank, blocks_per_rank);
 }
 
-template <typename T>
-__global__ void __launch_bounds__(simta::kThreadsShared, 2) sar_emul_simta_kernel(const __grid_constant__ SarEmulParams E, int blocks_per_rank) {
+template <typename T, int THREADS>
+__global__ void __launch_bounds__(THREADS, 512 / THREADS) sar_emul_simta_kernel(const __grid_constant__ SarEmulParams E, int blocks_per_rank) {
   __shared__ SarLaunchParams P;
   __shared__ simta::Shared S;
   load_rank_params(E, blockIdx.x / blocks_per_rank, P);
   if (!(P.participants >> P.rank & 1)) return;
-  run_rank_simta<T, simta::kThreadsShared>(P, blockIdx.x % blocks_per_rank, blocks_per_rank, S);
+  run_rank_simta<T, THREADS>(P, blockIdx.x % blocks_per_rank, blocks_per_rank, S);
 }
 
 template <typename T>
@@ -298,7 +298,7 @@ int sar_cuda_launch(const SarLaunchParams* p, int path, int blocks, int threads,
 }
 
 int sar_cuda_max_emulated_blocks(int dtype, int path, int threads) {
-  return sar_cuda_emulated_fit(dtype, path, threads, 0, SAR_MAX_OPS);
+  return sar_cuda_emulated_fit(dtype, path, path == SAR_PATH_SIMT ? threads : 0, 0, SAR_MAX_OPS);
 }
 
 int sar_cuda_emulated_fit(int dtype, int path, int threads, int stages, int num_ops) {
@@ -312,7 +312,9 @@ int sar_cuda_emulated_fit(int dtype, int path, int threads, int stages, int num_
       return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sar_emul_tma_kernel<T>, tma::kThreads, smem);
     }
     if (path == SAR_PATH_SIMTA)
-      return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sar_emul_simta_kernel<T>, simta::kThreadsShared, 0);
+      return threads == simta::kThreadsShared
+                 ? (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sar_emul_simta_kernel<T, simta::kThreadsShared>, simta::kThreadsShared, 0)
+                 : (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sar_emul_simta_kernel<T, simta::kThreads>, simta::kThreads, 0);
     return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sar_emul_simt_kernel<T>, threads <= 0 ? 512 : threads, 0);
   });
   return sms * per_sm;
@@ -346,7 +348,9 @@ int sar_cuda_launch_emulated(const SarLaunchParams* params, int n, int path, int
                                               args, smem, st);
     }
     if (path == SAR_PATH_SIMTA)
-      return (int)cudaLaunchCooperativeKernel((void*)sar_emul_simta_kernel<T>, dim3(n * blocks_per_rank), dim3(simta::kThreadsShared), args, 0, st);
+      return threads == simta::kThreadsShared
+                 ? (int)cudaLaunchCooperativeKernel((void*)sar_emul_simta_kernel<T, simta::kThreadsShared>, dim3(n * blocks_per_rank), dim3(simta::kThreadsShared), args, 0, st)
+                 : (int)cudaLaunchCooperativeKernel((void*)sar_emul_simta_kernel<T, simta::kThreads>, dim3(n * blocks_per_rank), dim3(simta::kThreads), args, 0, st);
     if (threads <= 0) threads = 512;
     return (int)cudaLaunchCooperativeKernel((void*)sar_emul_simt_kernel<T>, dim3(n * blocks_per_rank), dim3(threads), args, 0, st);
   });

@@ -22,7 +22,8 @@ int sar_cuda_launch(const struct SarLaunchParams* p, int path, int blocks, int t
 // n ranks emulated on the current device by ONE cooperative launch: params
 // points to n SarLaunchParams in host memory (read during the call), which
 // differ in rank, table, status, trace, delay and the caller's tensors only;
-// rank r is run by blocks [r*blocks_per_rank, (r+1)*blocks_per_rank).  Fails with
+// rank r is run by blocks [r*blocks_per_rank, (r+1)*blocks_per_rank).  On the simta path threads is 256 (two blocks
+// per SM) or anything else (512).  Fails with
 // cudaErrorCooperativeLaunchTooLarge when the blocks cannot all be resident.
 int sar_cuda_launch_emulated(const struct SarLaunchParams* params, int n, int path, int blocks_per_rank, int threads,
                              void* stream);
@@ -32,7 +33,7 @@ int sar_cuda_default_blocks(int path);
 int sar_cuda_pick_blocks(int path, uint64_t bytes);
 uint32_t sar_cuda_default_tile_bytes(int path);
 int sar_cuda_max_emulated_blocks(int dtype, int path, int threads);   // resident blocks on the current device
-// the same for a launch with `stages` ring stages (0: all; bulk-copy path) and tables of at most num_ops ops
+// the same for a launch of 256-thread blocks on the simta path (threads = 256), or with `stages` ring stages (0: all; bulk-copy path) and tables of at most num_ops ops
 int sar_cuda_emulated_fit(int dtype, int path, int threads, int stages, int num_ops);
 
 // Barrier across ranks on control channel `channel`: announces `epoch` and

@@ -119,7 +119,7 @@ static DevTable* upload(Rank& rk, const sar_table* t, int rank, char* err, int e
 // 8 ranks, fp32, against 4 blocks per rank: 25 MiB 742 -> 199 us, 256 MiB 7.68 -> 1.61 ms (one bulk-copy block per SM;
 // two since then, see tma::Shared); 6 ranks, simt, 12 MB 349 -> 70 us (76 us with 512 threads a block).
 static int emulated_blocks(sar_local_comm* c, const sar_program* prog, int dtype, int path, int* threads, int stages, uint64_t bytes) {
-  if (path == SAR_PATH_SIMT && *threads <= 0) *threads = 256;
+  if (path == SAR_PATH_SIMTA || (path == SAR_PATH_SIMT && *threads <= 0)) *threads = 256;
   cudaSetDevice(c->ranks[0].dev);   // occupancy is that of the current device
   int nops = 0;
   if (path == SAR_PATH_TMA)
@@ -228,7 +228,7 @@ int sar_local_run(sar_local_comm* c, const sar_program* prog, void* const* bufs,
   const uint32_t esize = dtype == SAR_F32 ? 4 : 2;
   const int path = o->path;
   int blocks = o->blocks > 0 ? o->blocks : sar_cuda_pick_blocks(path, count * esize);
-  int threads = o->threads, stages = o->stages;
+  int threads = path == SAR_PATH_SIMT ? o->threads : 0, stages = o->stages;
   if (c->emulate && o->blocks <= 0) {
     if (path == SAR_PATH_TMA && stages <= 0) stages = 3;   // two blocks per SM (see emulated_blocks)
     blocks = emulated_blocks(c, prog, dtype, path, &threads, stages, count * esize);
@@ -367,7 +367,7 @@ int sar_local_run(sar_local_comm* c, const sar_program* prog, void* const* bufs,
     for (int ph = 0; ph < nph; ++ph) {
       if (!(launches[ph].parts >> r & 1)) continue;
       if (delay_ns && delay_ns[r] && !delayed[r]) { CK((cudaError_t)sar_cuda_delay(delay_ns[r], rk.stream)); delayed[r] = true; }
-      CK((cudaError_t)sar_cuda_launch(&launches[ph].hp[r], path, launches[ph].blocks, o->threads, rk.stream));
+      CK((cudaError_t)sar_cuda_launch(&launches[ph].hp[r], path, launches[ph].blocks, threads, rk.stream));
     }
     if (o->timed) CK(cudaEventRecord(rk.ev1, rk.stream));
   }
