@@ -302,3 +302,24 @@ def test_default_launch_shape(n, count, staged, path):
         assert torch.equal(a, b)
         torch.testing.assert_close(a.double(), want, **TOL[torch.float32])
     comm.close()
+
+
+@pytest.mark.parametrize("count", [1, 3, 4, 8, 2047, 2048, 2049, 4096 + 7, 1_000_003])
+@pytest.mark.parametrize("offset", [0, 8, 1])   # elements: the vector path, 16-byte aligned again, and the scalar path
+def test_scale_cast_edges(count, offset):
+    """One product in fp32 and one rounding an element: equal bits, whatever the types, the ragged end or the alignment."""
+    from stragglar_b200 import ops
+    for a in (torch.float32, torch.bfloat16, torch.float16):
+        for b in (torch.float32, torch.bfloat16, torch.float16):
+            src = torch.randn(count + offset, device="cuda:0").to(a)[offset:]
+            guard = torch.full((count + offset + 16,), 7.0, device="cuda:0", dtype=b)
+            dst = guard[offset:offset + count]
+            ops.scale_cast(dst, src, 0.3)
+            torch.cuda.synchronize()
+            want = (src.float() * torch.tensor(0.3, dtype=torch.float32)).to(b)
+            assert torch.equal(dst, want), (a, b)
+            assert (guard[:offset] == 7.0).all() and (guard[offset + count:] == 7.0).all()
+            if a == b:
+                ops.scale_cast(src, src, 0.3)
+                torch.cuda.synchronize()
+                assert torch.equal(src, want)
