@@ -313,7 +313,7 @@ void ProcessGroupStragglar::device_barrier(Side& s) {
 }
 
 void ProcessGroupStragglar::run_program(Side& s, const sar::Program& prog, size_t data_off, uint64_t count,
-                                        at::ScalarType dtype, float scale, void* user, int user_dtype) {
+                                        at::ScalarType dtype, float scale, void* user, int user_dtype, void* lone) {
   Transport& t = *s.t;
   const int n = getSize(), me = getRank();
   const int dt = dtype_code(dtype);
@@ -324,11 +324,12 @@ void ProcessGroupStragglar::run_program(Side& s, const sar::Program& prog, size_
     if (!(c.participants >> me & 1)) continue;
     int blocks = t.cuda() ? (opts_.blocks > 0 ? opts_.blocks : sar_cuda_pick_blocks(opts_.path, count * esize)) : 1;
     if (t.cuda() && opts_.blocks <= 0 && c.blocks_hint > 0 && c.blocks_hint < blocks) blocks = c.blocks_hint;
-    if (t.cuda() && opts_.blocks <= 0 && n == 1 && blocks == 128) blocks = 148;   // a lone rank: one block per SM
+    uint32_t stages = (uint32_t)c.stages_hint;
+    if (t.cuda() && opts_.blocks <= 0 && n == 1) { stages = 0; blocks = sar_cuda_lone_blocks(opts_.path, count * esize, &stages); }
     const bool gated = c.gate_rounds && count * esize >= sar::gate_min_bytes();
     // staged launches poll a flag over the link for every tile they read from a peer, version 0 included: larger tiles
     const uint32_t tile_max = opts_.tile_bytes ? opts_.tile_bytes
-                            : (t.cuda() ? ((gated || user) ? sar::gate_tile_bytes() : sar_cuda_default_tile_bytes(opts_.path)) : (128u << 10));
+                            : (t.cuda() ? ((gated || (user && n > 1)) ? sar::gate_tile_bytes() : sar_cuda_default_tile_bytes(opts_.path)) : (128u << 10));
     const uint32_t tile_elems = sar::pick_tile_elems(count, esize, (uint32_t)c.num_chunks, (uint32_t)blocks, 2048, tile_max);
     const SarGeom g = sar::make_geom(count, esize, (uint32_t)c.num_chunks, tile_elems);
     TORCH_CHECK((uint64_t)g.tiles_per_chunk * g.num_chunks <= SAR_FLAG_CAPACITY, "tensor too large for the flag array");
@@ -351,7 +352,7 @@ void ProcessGroupStragglar::run_program(Side& s, const sar::Program& prog, size_
       for (int r = 0; r < n; ++r) {
         P.comm.flags[r] = t.flags(r, c.channel);
         P.comm.ctrl[r] = t.ctrl(r, c.channel);
-        P.comm.buf[r] = t.data(r) + data_off;
+        P.comm.buf[r] = lone ? lone : t.data(r) + data_off;
       }
       P.ops = (const SarOp*)it->second.first;
       P.round_begin = (const uint16_t*)it->second.second;
@@ -369,10 +370,15 @@ void ProcessGroupStragglar::run_program(Side& s, const sar::Program& prog, size_
       }
       P.gate_rounds = gated ? 1u : 0u;
       P.gate_base = epoch64; P.gate_slack = sar::gate_slack(g.tiles_per_chunk);
-      P.stages = (uint32_t)c.stages_hint;
+      P.stages = stages;
       P.lane1_eighths = (uint32_t)c.lane1_eighths;
       int launch_blocks = blocks;
-      if (user) {
+      if (user && n == 1) {
+        // The rank's own memory is the only bound, and every tile stays with one block from copy-in to copy-out.
+        // (With a staging block on top of the 148 of a large tensor the launch did not fit the device, and the blocks
+        // that were resident waited for the one that was not until the wait ran out.)
+        P.staging_blocks = SAR_STAGE_EVERYWHERE;
+      } else if (user) {
         // staging blocks on top of the table's: local copies need many blocks to run at memory speed
         const int extra = std::max(1, std::min(64, 144 - blocks));
         P.staging_blocks = (uint32_t)extra;
@@ -469,6 +475,12 @@ void ProcessGroupStragglar::allreduce_impl(Side& s, at::Tensor& tensor, float sc
   if (opts_.check_args) check_same_arguments(count, dtype_code(tdt), cdc, (hoff >= 0 && (((uintptr_t)ptr) & 15) == 0) ? hoff : -1);
   if (hoff >= 0 && (((uintptr_t)ptr) & 15) == 0) {
     run_program(s, prog, (size_t)hoff, count, cdt, scale);   // in place, no staging
+    return;
+  }
+  if (t.cuda() && getSize() == 1 && cdt == tdt && (((uintptr_t)ptr) & 15) == 0) {
+    // A group of one has no peers that would have to reach the tensor: in place as well, one pass over it instead of
+    // three (in, scale, out).
+    run_program(s, prog, 0, count, cdt, scale, nullptr, 0, ptr);
     return;
   }
   const size_t tsize = tensor.element_size();

@@ -820,6 +820,25 @@ __device__ void simt_tile(const SarLaunchParams& P, const Item& it, const uint32
         st_vec(own + (size_t)v * 16, o);
         if (push) st_vec(push + (size_t)v * 16, o);
       }
+    } else if (nsrc == 0) {
+      // a lone rank scales its buffer in place: nothing to add, so twice the vectors in flight
+      // (1 GiB fp32 with one vector at a time: 647 to 775 us, depending on the tile; now 366)
+      auto scaled = [&](uint4 r) {
+        float f[N];
+        Vec<T>::unpack(r, f);
+#pragma unroll
+        for (int i = 0; i < N; ++i) f[i] = (local ? f[i] : 0.0f) * scale;
+        return Vec<T>::pack(f);
+      };
+      uint32_t v = tid;
+      for (; v + (2 * UNROLL - 1) * nth < nvec; v += 2 * UNROLL * nth) {
+        uint4 r[2 * UNROLL];
+#pragma unroll
+        for (int u = 0; u < 2 * UNROLL; ++u) r[u] = ld_vec_sys(own + (size_t)(v + u * nth) * 16);
+#pragma unroll
+        for (int u = 0; u < 2 * UNROLL; ++u) st_vec(own + (size_t)(v + u * nth) * 16, scaled(r[u]));
+      }
+      for (; v < nvec; v += nth) st_vec(own + (size_t)v * 16, scaled(ld_vec_sys(own + (size_t)v * 16)));
     } else {
       // several peers (reduce-scatter stage): all sources of a vector in flight at once
       for (uint32_t v = tid; v < nvec; v += nth) {

@@ -233,7 +233,11 @@ int sar_local_run(sar_local_comm* c, const sar_program* prog, void* const* bufs,
     if (path == SAR_PATH_TMA && stages <= 0) stages = 3;   // two blocks per SM (see emulated_blocks)
     blocks = emulated_blocks(c, prog, dtype, path, &threads, stages, count * esize);
   }
-  if (n == 1 && o->blocks <= 0 && blocks == 128) blocks = 148;   // a lone rank streams its own memory: one block per SM
+  if (n == 1 && !c->emulate && o->blocks <= 0) {
+    uint32_t st = stages > 0 ? (uint32_t)stages : 0u;
+    blocks = sar_cuda_lone_blocks(path, count * esize, &st);
+    stages = (int)st;
+  }
   const double timeout_s = o->timeout_s > 0 ? o->timeout_s : 10.0;
   // Emulated ranks, simt and simta: tiles of up to 256 KiB, because the wait, the block barriers and the fence around
   // a tile are not hidden behind another one (ring, 4 ranks, 40 MB: 124 us against 137 with 128 KiB; level where the
@@ -313,7 +317,7 @@ int sar_local_run(sar_local_comm* c, const sar_program* prog, void* const* bufs,
       if (o->user_in && o->user_out) {
         P.user_in = o->user_in[r]; P.user_out = o->user_out[r]; P.user_dtype = o->user_dtype;
         sar_table_final_ver(t, r, P.final_ver);
-        if (c->emulate && o->blocks <= 0) P.staging_blocks = SAR_STAGE_EVERYWHERE;
+        if ((c->emulate || n == 1) && o->blocks <= 0) P.staging_blocks = SAR_STAGE_EVERYWHERE;
       }
       P.delay_ns = 0;
       if (c->emulate && delay_ns && delay_ns[r] && !delayed[r] && (parts >> r & 1)) { P.delay_ns = delay_ns[r]; delayed[r] = true; }

@@ -89,6 +89,33 @@ def test_backend_world1_on_one_gpu():
     run_ranks(1, _cuda_collectives)
 
 
+def _lone_rank(rank, world):
+    import stragglar_b200.parallel as sp
+    torch.cuda.set_device(rank)
+    dev = torch.device("cuda", rank)
+    # one block's worth, ragged, around one block per ring stage, and more blocks than SMs (also in staged mode)
+    for count in (1, 5, 8 * 1024 + 1, 1 << 20, 9 * (1 << 20) + 3, 34 * (1 << 20) + 1):
+        g = torch.Generator(device=dev).manual_seed(count)
+        x = torch.empty(count + 1, device=dev).normal_(generator=g)
+        for dtype, off, wire in ((torch.float32, 0, None), (torch.bfloat16, 0, None), (torch.float32, 1, None),
+                                 (torch.float32, 0, torch.bfloat16), (torch.bfloat16, 0, torch.float32)):
+            t = x.to(dtype)[off:off + count]
+            want = t.clone() if wire is None else t.to(wire).to(dtype)   # the mean of one rank, rounded once to the wire
+            if wire is None:
+                dist.all_reduce(t, op=dist.ReduceOp.AVG)
+            else:
+                sp.all_reduce_ex(t, average=True, comm_dtype=wire).wait()
+            assert torch.equal(t, want), (count, dtype, off, wire)
+    torch.cuda.synchronize()
+    assert sp.check_status(dev) == 0 and sp.check_guards(dev)
+
+
+def test_lone_rank_of_every_size():
+    """A group of one: symmetric or not, aligned or not, converted or not, up to sizes whose staged launch used to need
+    more blocks than fit the device at once."""
+    run_ranks(1, _lone_rank)
+
+
 @pytest.mark.multigpu
 def test_backend_on_all_gpus():
     world = min(torch.cuda.device_count(), 8)
