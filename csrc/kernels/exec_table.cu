@@ -302,7 +302,10 @@ int sar_cuda_lone_blocks(int path, uint64_t bytes, uint32_t* stages) {
 }
 uint32_t sar_cuda_default_tile_bytes(int path) { return path == SAR_PATH_TMA ? (64u << 10) : (128u << 10); }
 
-int sar_cuda_launch(const SarLaunchParams* p, int path, int blocks, int threads, void* stream) {
+int sar_cuda_launch(const SarLaunchParams* params, int path, int blocks, int threads, void* stream) {
+  SarLaunchParams filled = *params;
+  sar_fill_chunks(&filled);
+  const SarLaunchParams* p = &filled;
   if (blocks <= 0) blocks = sar_cuda_default_blocks(path);
   cudaStream_t st = (cudaStream_t)stream;
   return with_dtype(p->dtype, [&](auto tag) -> int {
@@ -353,6 +356,7 @@ int sar_cuda_launch_emulated(const SarLaunchParams* params, int n, int path, int
   cudaStream_t st = (cudaStream_t)stream;
   SarEmulParams E;
   E.common = params[0];
+  sar_fill_chunks(&E.common);
   memset(E.rank, 0, sizeof E.rank);
   for (int r = 0; r < n; ++r) {
     const SarLaunchParams& P = params[r];

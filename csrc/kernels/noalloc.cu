@@ -140,6 +140,7 @@ extern "C" int sar_emulated_allreduce_noalloc(const sar_table* table, void* cons
     P.epoch_base = SAR_VER_STRIDE; P.scale = scale; P.dtype = dtype;
     P.timeout_ns = 10000000000ull;
     P.status = device_status; P.trace = nullptr; P.delay_ns = 0;
+    sar_fill_chunks(&P);
   }
   e = cudaMemcpyAsync(S + kParamsOff, hp, sizeof(SarLaunchParams) * n, cudaMemcpyHostToDevice, st);
   if (e != cudaSuccess) return fail(err, errlen, (int)e, cudaGetErrorString(e));

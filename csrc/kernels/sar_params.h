@@ -60,11 +60,20 @@ struct SarLaunchParams {
                            // SAR_STAGE_EVERYWHERE: every block stages its share in, walks the table, stages out
   uint64_t delay_ns;      // spin this long before arriving (a late rank when ranks share one launch)
   SarMcGroup mc[2];       // multicast views (simt path): all ranks, and e.g. the non-stragglers
+  // The chunks of `geom`, worked out on the host (sar_fill_chunks; the launchers do it): every block needs them before
+  // it can start and for every staging item, and a 64-bit division costs a thread some hundred cycles.
+  uint64_t chunk_begin[SAR_MAX_CHUNKS + 1];
+  uint32_t chunk_tiles[SAR_MAX_CHUNKS];
 };
+inline void sar_fill_chunks(SarLaunchParams* p) {
+  for (uint32_t c = 0; c <= SAR_MAX_CHUNKS; ++c) p->chunk_begin[c] = c < p->geom.num_chunks ? sar_chunk_begin(p->geom, c) : p->geom.count;
+  for (uint32_t c = 0; c < SAR_MAX_CHUNKS; ++c)
+    p->chunk_tiles[c] = (uint32_t)((p->chunk_begin[c + 1] - p->chunk_begin[c] + p->geom.tile_elems - 1) / p->geom.tile_elems);
+}
 
 
 // Launch parameters of n ranks emulated on one device: what the ranks share once, and per rank what differs.  Passed
-// to the kernel by value (2.7 KB of the 32 KB a launch may carry), so a collective is one launch and no copy.
+// to the kernel by value (3 KB of the 32 KB a launch may carry), so a collective is one launch and no copy.
 // (With a copy to device memory ahead of the launch, start to end on the stream was 3 us longer.)
 struct SarEmulRank {
   const SarOp* ops;
