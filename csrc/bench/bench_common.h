@@ -40,7 +40,7 @@ struct Options {
   int straggler = -1;      // STRAGGLAR_STRAGGLER: physical rank that is late (default n-1)
   int path = SAR_PATH_SIMT;// STRAGGLAR_PATH = simt | tma | simta
   int blocks = 0, threads = 0;
-  int store_window = 0;    // STRAGGLAR_STORE_WINDOW: store groups a block keeps in flight on the bulk-copy path (3, 8, 16)
+  int store_window = 0;    // STRAGGLAR_STORE_WINDOW: accepted and without effect (see sar_run_opts)
   int stages = 0;          // STRAGGLAR_STAGES: ring stages per block on the bulk-copy path (0: all)
   uint32_t tile_bytes = 0;
   double timeout_s = 10.0; // STRAGGLAR_TIMEOUT_MS

@@ -15,7 +15,7 @@ __global__ void __launch_bounds__(512, 1) sar_exec_simt_kernel(const __grid_cons
 }
 
 template <typename T>
-__global__ void __launch_bounds__(tma::kThreads, 1) sar_exec_tma_kernel(const __grid_constant__ SarLaunchParams P) {
+__global__ void __launch_bounds__(tma::kThreads, 2) sar_exec_tma_kernel(const __grid_constant__ SarLaunchParams P) {
   run_rank_tma<T>(P, blockIdx.x, gridDim.x, *reinterpret_cast<tma::Shared*>(sar_smem));
 }
 
@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) sar_emul_simta_kernel(
 }
 
 template <typename T>
-__global__ void __launch_bounds__(tma::kThreads, 1) sar_emul_tma_kernel(const __grid_constant__ SarEmulParams E, int blocks_per_rank) {
+__global__ void __launch_bounds__(tma::kThreads, 2) sar_emul_tma_kernel(const __grid_constant__ SarEmulParams E, int blocks_per_rank) {
   __shared__ SarLaunchParams P;
   load_rank_params(E, blockIdx.x / blocks_per_rank, P);
   if (!(P.participants >> P.rank & 1)) return;

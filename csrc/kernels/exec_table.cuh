@@ -15,10 +15,11 @@
 //   * simt: every thread moves 16-byte vectors with ld.relaxed.sys / st;
 //   * tma:  a producer thread streams tiles from peer memory into a shared
 //           memory ring with bulk async copies (cp.async.bulk + mbarrier
-//           complete_tx), consumer warps add in place, bulk stores write the
-//           result to local and peer memory, and a signal thread announces
-//           finished tiles, keeping the system-scope fence off the issue path.
-//           Few threads keep hundreds of KB in flight per block.
+//           complete_tx), consumer warps add in place, and storer threads
+//           write the result to local and peer memory with bulk stores and
+//           announce finished tiles, keeping the wait for the stores and the
+//           fence off the issue path.  Few threads keep hundreds of KB in
+//           flight per block.
 //
 // Every wait (peer arrival, tile flag, pipeline barrier, exit) is bounded by a
 // %globaltimer deadline.  On expiry the block records a SarStatus, raises the
@@ -989,8 +990,11 @@ namespace tma {
 constexpr int kStages = 6;
 constexpr int kStageBytes = 32768;
 constexpr int kConsumerWarps = 4;
-constexpr int kThreads = 32 * (2 + kConsumerWarps);   // producer warp, consumer warps, signal warp
-constexpr int kPendRing = 32;
+constexpr int kStorers = 3;
+constexpr int kThreads = 32 * (1 + kConsumerWarps + kStorers);   // producer warp, consumer warps, storing warps
+constexpr int kQueue = 8;                                        // at least every stage's piece and the end marker
+constexpr uint32_t kQueueEnd = 0xffffffffu;
+static_assert(kQueue > kStages, "a storer's queue holds whatever the ring holds");
 
 struct StageDesc {
   const SarOp* op;      // nullptr: no more work
@@ -1011,25 +1015,23 @@ struct StageDesc {
   uint64_t dst_off;     // byte offset on the destination side
   uint32_t piece_elems; // elements in this piece
 };
-struct PendEntry { const SarOp* op; uint32_t fidx; uint32_t seq; };
 
 // Dynamic shared memory of a block: this structure, the op table (ops_offset), and the ring of `stages` stages
 // (ring_offset).  A launch that asks for fewer than kStages stages may allocate just those.
 // Ranks on one device: a block is a serial chain (wait, load, add, store, announce) at some 27 GB/s, whatever its ring
 // holds, so two blocks with three stages each share an SM instead of one with six.  8 ranks, fp32: 25 MiB 206 -> 141 us,
-// 256 MiB 1634 -> 1137 us, a staged 25 MiB bucket 464 -> 323 us.  Three blocks with two stages: 195 us at 25 MiB (a
-// stage is handed back one piece late, which leaves a ring of two with nothing in flight).
+// 256 MiB 1634 -> 1137 us, a staged 25 MiB bucket 464 -> 323 us.  Since a stage is handed back as soon as it is stored
+// (run_rank_tma): 123 us at 25 MiB, against 133 with three blocks of two stages and 130 to 155 with stages of 16 or
+// 24 KiB and as many blocks as fit.
 struct Shared {
-  alignas(8) uint64_t full[kStages];
-  alignas(8) uint64_t empty[kStages];
+  alignas(8) uint64_t full[kStages];    // the piece's loads have landed (and its descriptor is written)
+  alignas(8) uint64_t added[kStages];   // every consumer warp is done with the piece
+  alignas(8) uint64_t empty[kStages];   // ... and its storer too: the stage may be refilled
   StageDesc desc[kStages];
   TableGeom geom;
-  // finished items on their way to the signal warp
-  PendEntry pend[kPendRing];
-  uint32_t pend_tail;   // written by the storing thread
-  uint32_t pend_head;   // written by the signal thread
-  uint32_t landed;      // store groups with seq < landed have completed
-  uint32_t consumers_done;
+  // pieces on their way to the storers: an item goes to one storer, items are dealt in turn
+  uint32_t queue[kStorers][kQueue];     // sequence numbers of pieces, kQueueEnd after the last one
+  uint32_t queue_tail[kStorers];        // written by the producer
   int abort_seen;
   uint32_t issued;      // pieces the producer has issued (written when it stops)
 };
@@ -1057,17 +1059,6 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* b, uint32_t parity) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(b)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-__device__ __forceinline__ bool mbar_test_wait(uint64_t* b, uint32_t parity) {   // never suspends the thread
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(ok)
       : "r"(smem_u32(b)), "r"(parity)
@@ -1102,7 +1093,6 @@ template <int N> __device__ __forceinline__ void bulk_wait_read() {
 template <int N> __device__ __forceinline__ void bulk_wait_all() {
   asm volatile("cp.async.bulk.wait_group %0;" ::"n"(N) : "memory");
 }
-__device__ __forceinline__ void consumer_bar() { asm volatile("bar.sync 1, %0;" ::"n"(32 * kConsumerWarps) : "memory"); }
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void fence_proxy_async_global() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
 __device__ __forceinline__ uint32_t ld_acquire_cta(const uint32_t* p) {
@@ -1183,14 +1173,22 @@ __device__ void convert_piece(unsigned char* dst, int ddt, const unsigned char* 
   }
 }
 
-// Roles of a block (192 threads):
-//   warp 0, one thread   producer: walks the items, waits for their operands
-//                        (flags in peer memory), streams the tiles into the ring;
-//   warps 1-4            consumers: add the sources of a stage in place; one of
-//                        their threads issues the bulk stores and recycles stages;
-//   warp 5, one thread   signal: announces finished items (fence + flag stores).
-// Announcing costs a system-scope fence; doing it in a thread of its own keeps
-// the fence off the path that issues loads and stores.
+// Roles of a block (256 threads):
+//   warp 0, one thread     producer: walks the items, waits for their operands
+//                          (flags in peer memory), streams the tiles into the ring;
+//   warps 1-4              consumers: add (or convert) the sources of a stage in place;
+//   warps 5-7, one thread  storers: issue the bulk stores of their items' pieces, hand
+//                          each stage back as soon as its store has read it, and when an
+//                          item's stores have completed announce it (fence + flag stores).
+// Completion of bulk stores can only be waited for, and announcing costs a fence: a
+// storer spends that time on its own item while the others keep storing, so the
+// latency of neither is on the path that loads, adds or recycles stages.  Before, one
+// consumer thread stored, handed a stage back one piece late, let three stores be in
+// flight and told a signal thread what had landed when a store left that window or the
+// pipeline ran dry.  8 ranks on one device: 256 MiB fp32 1034 -> 961 us, 25 MiB 137 ->
+// 122 us, bf16-wire bucket 179 -> 157 us, 1 MiB bf16 stragglar_a2a 39.7 -> 37.7 us;
+// 4-rank ring, 40 MB 108 -> 95 us.  (Handing stages back at once from the consumer
+// thread instead: 1001 us, but 143 us at 25 MiB.)
 template <typename T>
 __device__ void run_rank_tma(const SarLaunchParams& P, uint32_t block, uint32_t nblocks, tma::Shared& S) {
   using namespace tma;
@@ -1202,9 +1200,11 @@ __device__ void run_rank_tma(const SarLaunchParams& P, uint32_t block, uint32_t 
   OpGeom* const op_mem = reinterpret_cast<OpGeom*>(reinterpret_cast<unsigned char*>(&S) + ops_offset());
   WaitCtx w = enter_collective(P, block);
   if (tid == 0) {
-    for (int s = 0; s < kStages; ++s) { mbar_init(&S.full[s], 1); mbar_init(&S.empty[s], 1); }
+    for (int s = 0; s < kStages; ++s) {
+      mbar_init(&S.full[s], 1); mbar_init(&S.added[s], kConsumerWarps); mbar_init(&S.empty[s], kConsumerWarps + 1);
+    }
     S.abort_seen = 0; S.issued = 0;
-    S.pend_tail = 0; S.pend_head = 0; S.landed = 0; S.consumers_done = 0;
+    for (int k = 0; k < kStorers; ++k) S.queue_tail[k] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     fence_proxy_async();
   }
@@ -1218,8 +1218,17 @@ __device__ void run_rank_tma(const SarLaunchParams& P, uint32_t block, uint32_t 
       walk.init(&P, &S.geom, block, nblocks);
       uint32_t arrived = 1u << P.rank, gate_passed = 0;
       uint32_t seq = 0;           // pieces issued
+      uint32_t storer = kStorers - 1, tails[kStorers] = {};
       bool ok = true;
       Item it;
+      auto hand_over = [&](uint32_t what) {       // to the item's storer
+#pragma unroll
+        for (int k = 0; k < kStorers; ++k)
+          if ((uint32_t)k == storer) {
+            S.queue[k][tails[k] % kQueue] = what;
+            st_release_cta(&S.queue_tail[k], ++tails[k]);
+          }
+      };
       auto acquire_stage = [&](uint32_t s) -> bool {
         // the first pass over the ring finds every stage free
         if (seq >= nst) return mbar_wait(&S.empty[s], ((seq / nst) - 1) & 1, w);
@@ -1231,6 +1240,7 @@ __device__ void run_rank_tma(const SarLaunchParams& P, uint32_t block, uint32_t 
         if (P.trace_rounds) trace_item_start(P, it.op, t_begin, globaltimer());
         fence_proxy_async_global();   // flags were acquired through the generic proxy; the copies use the async one
         const SarOp* op = it.op;
+        storer = storer + 1 == kStorers ? 0 : storer + 1;
         if (op->kind >= SAR_STAGE_IN) {
           const bool in = op->kind == SAR_STAGE_IN;
           const int sdt = in ? P.user_dtype : P.dtype, ddt = in ? P.dtype : P.user_dtype;
@@ -1245,6 +1255,7 @@ __device__ void run_rank_tma(const SarLaunchParams& P, uint32_t block, uint32_t 
             d.op = op; d.byte_off = 0; d.bytes = 0; d.slot_bytes = 0; d.nsrc_total = 0; d.fidx = it.fidx; d.last = 1u;
             d.tail_elems = 0; d.tail_elem0 = 0; d.item_elem0 = it.elem0; d.item_elems = it.nelem; d.dst_bytes = 0;
             mbar_arrive(&S.full[s]);
+            hand_over(seq);
             ++seq;
             continue;
           }
@@ -1270,6 +1281,7 @@ __device__ void run_rank_tma(const SarLaunchParams& P, uint32_t block, uint32_t 
             } else {
               mbar_arrive(&S.full[s]);
             }
+            hand_over(seq);
             ++seq;
             done += pe;
           } while (done < body);
@@ -1302,6 +1314,7 @@ __device__ void run_rank_tma(const SarLaunchParams& P, uint32_t block, uint32_t 
           } else {
             mbar_arrive(&S.full[s]);   // an item that is only a sub-vector tail
           }
+          hand_over(seq);
           ++seq;
           done += bytes;
         } while (done < vec_bytes);
@@ -1317,6 +1330,7 @@ __device__ void run_rank_tma(const SarLaunchParams& P, uint32_t block, uint32_t 
         if (got) { S.desc[s].op = nullptr; mbar_arrive(&S.full[s]); }
         else *(volatile int*)&S.abort_seen = 1;
       }
+      for (storer = 0; storer < (uint32_t)kStorers; ++storer) hand_over(kQueueEnd);
       S.issued = seq;
     }
   } else if (warp <= (uint32_t)kConsumerWarps) {
@@ -1324,20 +1338,10 @@ __device__ void run_rank_tma(const SarLaunchParams& P, uint32_t block, uint32_t 
     const uint32_t ctid = tid - 32;                 // 0 .. 127
     constexpr uint32_t CT = 32 * kConsumerWarps;
     uint32_t seq = 0;
-    uint32_t landed = 0, pend_tail = 0;             // private copies of the storing thread (ctid 0)
-    const uint32_t win = P.store_window >= 16 ? 16u : (P.store_window >= 8 ? 8u : 3u);
     while (true) {
       const uint32_t s = seq % nst;
       bool ok = true;
       if (lane == 0) {
-        if (ctid == 0 && landed < seq && !mbar_test_wait(&S.full[s], (seq / nst) & 1)) {
-          // The pipeline has run dry, perhaps because the producer waits for a tile
-          // that (through other ranks) depends on an item whose stores have not been
-          // reported as landed yet: report everything now.
-          bulk_wait_all<0>();
-          landed = seq;
-          st_release_cta(&S.landed, landed);
-        }
         ok = mbar_wait(&S.full[s], (seq / nst) & 1, w);
         if (*(volatile int*)&S.abort_seen) ok = false;
       }
@@ -1399,89 +1403,65 @@ __device__ void run_rank_tma(const SarLaunchParams& P, uint32_t block, uint32_t 
         }
         fence_proxy_async_smem();   // make the sums visible to the bulk store engine
       }
-      // Every consumer warp is done with this piece's descriptor and data, and
-      // (a fortiori) with the previous piece's stage, which is released below.
-      consumer_bar();
-      if (ctid == 0) {
-        if (op->kind >= SAR_STAGE_IN) {
-          if (d.dst_bytes) {
-            char* dst = op->kind == SAR_STAGE_IN ? (char*)P.comm.buf[P.rank] : (char*)P.user_out;
-            bulk_store(dst + d.dst_off, d.bytes != d.dst_bytes ? stage + kStageBytes / 2 : stage, d.dst_bytes);
-          }
-        } else if (d.bytes) {
-          if (op->kind != SAR_PUSH) bulk_store((char*)P.comm.buf[P.rank] + d.byte_off, stage, d.bytes);
-          if (op->kind == SAR_REDUCE_PUSH) bulk_store((char*)P.comm.buf[op->src[0]] + d.byte_off, stage, d.bytes);
-          if (op->kind == SAR_PUSH)
-            for (int q = 0; q < op->nsrc; ++q) bulk_store((char*)P.comm.buf[op->src[q]] + d.byte_off, stage, d.bytes);
-        }
-        bulk_commit();          // one group per piece (possibly empty), so group numbers follow seq
-        if (d.last) {
-          if (d.tail_elems && op->kind >= SAR_STAGE_IN) {
-            const bool in = op->kind == SAR_STAGE_IN;
-            const void* tsrc = in ? P.user_in : (const void*)P.comm.buf[P.rank];
-            void* tdst = in ? (void*)P.comm.buf[P.rank] : P.user_out;
-            for (uint32_t i = 0; i < d.tail_elems; ++i)
-              store_from_float(tdst, d.tail_elem0 + i, in ? P.dtype : P.user_dtype, load_as_float(tsrc, d.tail_elem0 + i, in ? P.user_dtype : P.dtype));
-            __threadfence_system();
-          } else if (d.tail_elems) { scalar_elems<T>(P, op, d.tail_elem0, d.tail_elems); __threadfence_system(); }
-          // hand the item to the signal thread; wait (bounded) if its ring is full
-          if (pend_tail - ld_acquire_cta(&S.pend_head) >= (uint32_t)kPendRing) {
-            bulk_wait_all<0>();
-            landed = seq + 1;
-            st_release_cta(&S.landed, landed);
-            while (pend_tail - ld_acquire_cta(&S.pend_head) >= (uint32_t)kPendRing) {
-              if (*(volatile uint32_t*)w.abort_flag || globaltimer() > w.deadline) break;
-            }
-          }
-          PendEntry& e = S.pend[pend_tail % kPendRing];
-          e.op = op; e.fidx = d.fidx; e.seq = seq;
-          ++pend_tail;
-          st_release_cta(&S.pend_tail, pend_tail);
-        }
-        // the previous piece's stores have read their stage: hand it back
-        bulk_wait_read<1>();
-        if (seq >= 1) mbar_arrive(&S.empty[(seq - 1) % nst]);
-        // at most `win` store groups stay in flight; older ones have landed.  Stores to peer memory are
-        // posted: a deep window keeps a block's pushes from being paced by the link's round trip.
-        if (win >= 16) bulk_wait_all<16>();
-        else if (win >= 8) bulk_wait_all<8>();
-        else bulk_wait_all<3>();
-        if (seq >= win && landed < seq - (win - 1)) { landed = seq - (win - 1); st_release_cta(&S.landed, landed); }
-      }
+      __syncwarp();
+      if (lane == 0) { mbar_arrive(&S.added[s]); mbar_arrive(&S.empty[s]); }
       ++seq;
     }
-    if (ctid == 0) {
-      bulk_wait_all<0>();
-      st_release_cta(&S.landed, 0xffffffffu);
-      st_release_cta(&S.consumers_done, 1u);
-    }
   } else if (lane == 0) {
-    // ------------------------------------------------------------------ signal
-    uint32_t head = 0;
-    while (true) {
-      const uint32_t done = ld_acquire_cta(&S.consumers_done);
-      const uint32_t tail = ld_acquire_cta(&S.pend_tail);
-      const uint32_t landed = ld_acquire_cta(&S.landed);
-      uint32_t n = 0;
-      while (head + n != tail && S.pend[(head + n) % kPendRing].seq < landed) ++n;
-      if (n) {
-        fence_proxy_async_global();   // the tiles were written by bulk copies
-        fence_ranks(w.one_device);
-        for (uint32_t i = 0; i < n; ++i) {
-          const PendEntry& e = S.pend[(head + i) % kPendRing];
-          publish_item(P, e.op, e.fidx);
-          trace_item_end(P, e.op);
-          gate_item_done(P, S.geom, e.op);
-        }
-        head += n;
-        st_release_cta(&S.pend_head, head);
-        continue;
+    // ----------------------------------------------------------------- storers
+    const uint32_t k = warp - 1 - kConsumerWarps;
+    for (uint32_t head = 0;; ++head) {
+      bool more = true;
+      for (uint32_t it = 0; ld_acquire_cta(&S.queue_tail[k]) == head; ++it) {
+        if ((it & 63) == 63 && globaltimer() > w.deadline + 1000000000ull) { more = false; break; }   // the producer is long gone
+        __nanosleep(20);
       }
-      if (done && head == tail) break;
-      if (*(volatile uint32_t*)w.abort_flag && done) break;
-      if (globaltimer() > w.deadline + 1000000000ull) break;   // the other roles have given up long ago
-      __nanosleep(w.one_device ? 20 : 64);
+      if (!more) break;
+      const uint32_t seq = S.queue[k][head % kQueue];
+      if (seq == kQueueEnd) break;
+      const uint32_t s = seq % nst, parity = (seq / nst) & 1;
+      const StageDesc& d = S.desc[s];       // the stage stays this piece's until it is handed back below
+      const SarOp* op = d.op;
+      const bool copied = op->kind == SAR_COPY || op->kind == SAR_PUSH;      // nothing to add: from the loads to the stores
+      if (!mbar_wait(copied ? &S.full[s] : &S.added[s], parity, w)) break;
+      const unsigned char* stage = ring + s * kStageBytes;
+      if (op->kind >= SAR_STAGE_IN) {
+        if (d.dst_bytes) {
+          char* dst = op->kind == SAR_STAGE_IN ? (char*)P.comm.buf[P.rank] : (char*)P.user_out;
+          bulk_store(dst + d.dst_off, d.bytes != d.dst_bytes ? stage + kStageBytes / 2 : stage, d.dst_bytes);
+        }
+      } else if (d.bytes) {
+        if (op->kind != SAR_PUSH) bulk_store((char*)P.comm.buf[P.rank] + d.byte_off, stage, d.bytes);
+        if (op->kind == SAR_REDUCE_PUSH) bulk_store((char*)P.comm.buf[op->src[0]] + d.byte_off, stage, d.bytes);
+        if (op->kind == SAR_PUSH)
+          for (int q = 0; q < op->nsrc; ++q) bulk_store((char*)P.comm.buf[op->src[q]] + d.byte_off, stage, d.bytes);
+      }
+      bulk_commit();
+      const bool last = d.last != 0;
+      const uint32_t fidx = d.fidx;
+      if (last && d.tail_elems) {
+        if (op->kind >= SAR_STAGE_IN) {
+          const bool in = op->kind == SAR_STAGE_IN;
+          const void* tsrc = in ? P.user_in : (const void*)P.comm.buf[P.rank];
+          void* tdst = in ? (void*)P.comm.buf[P.rank] : P.user_out;
+          for (uint32_t i = 0; i < d.tail_elems; ++i)
+            store_from_float(tdst, d.tail_elem0 + i, in ? P.dtype : P.user_dtype, load_as_float(tsrc, d.tail_elem0 + i, in ? P.user_dtype : P.dtype));
+        } else {
+          scalar_elems<T>(P, op, d.tail_elem0, d.tail_elems);
+        }
+      }
+      bulk_wait_read<0>();                  // the stores have read the stage
+      mbar_arrive(&S.empty[s]);
+      if (last && op->kind != SAR_STAGE_OUT) {
+        bulk_wait_all<0>();
+        fence_proxy_async_global();         // the tile was written by bulk copies
+        fence_ranks(w.one_device);
+        publish_item(P, op, fidx);
+        trace_item_end(P, op);
+        gate_item_done(P, S.geom, op);
+      }
     }
+    bulk_wait_all<0>();
   }
   __syncthreads();
   // Bulk loads still in flight would write into shared memory after the block
@@ -1514,6 +1494,7 @@ constexpr int kThreads = 512;
 constexpr int kThreadsShared = 256;   // ranks on one device: two blocks per SM (see run_rank_simta)
 constexpr int kSlots = 2;
 constexpr int kPendRing = 16;
+struct PendEntry { const SarOp* op; uint32_t fidx; };   // a finished item on its way to the signal thread
 
 struct Shared {
   TableGeom geom;
@@ -1524,7 +1505,7 @@ struct Shared {
   int decision;               // the state the workers act on (written by worker thread 0)
   alignas(8) uint64_t full[kSlots];
   alignas(8) uint64_t empty[kSlots];
-  tma::PendEntry pend[kPendRing];
+  PendEntry pend[kPendRing];
   uint32_t pend_tail;         // written by worker thread 0
   uint32_t pend_head;         // written by the signal thread
   uint32_t workers_done;
@@ -1575,8 +1556,8 @@ __device__ void run_rank_simta(const SarLaunchParams& P, uint32_t block, uint32_
         while (pend_tail - ld_acquire_cta(&S.pend_head) >= (uint32_t)kPendRing) {
           if (*(volatile uint32_t*)w.abort_flag || globaltimer() > w.deadline) break;
         }
-        tma::PendEntry& e = S.pend[pend_tail % kPendRing];
-        e.op = it.op; e.fidx = it.fidx; e.seq = seq;
+        PendEntry& e = S.pend[pend_tail % kPendRing];
+        e.op = it.op; e.fidx = it.fidx;
         ++pend_tail;
         st_release_cta(&S.pend_tail, pend_tail);
         mbar_arrive(&S.empty[s]);
@@ -1620,7 +1601,7 @@ __device__ void run_rank_simta(const SarLaunchParams& P, uint32_t block, uint32_
       if (head != tail) {
         fence_ranks(w.one_device);     // the tiles' stores (ordered before the hand-off) become visible first
         for (; head != tail; ++head) {
-          const tma::PendEntry& e = S.pend[head % kPendRing];
+          const PendEntry& e = S.pend[head % kPendRing];
           publish_item(P, e.op, e.fidx);
           trace_item_end(P, e.op);
           gate_item_done(P, S.geom, e.op);

@@ -45,7 +45,6 @@ struct SarLaunchParams {
   uint32_t gate_slack;    // round gating: items of a round that may still be running when the next round opens
   uint64_t gate_base;     // round gating: value that stands for round 0 of this launch (grows by >= 32 per launch)
   uint32_t stages;        // bulk-copy path: ring stages in use (0 or > the ring size: all)
-  uint32_t store_window;  // bulk-copy path: store groups a block keeps in flight (3, 8 or 16; 0: 3)
   // Staged mode (all three null/zero: off).  The caller's tensor is not reachable by peers: the kernel itself copies
   // it tile by tile into this rank's buffer before the table's ops (announcing every tile as version 0 through its
   // flag, so that nobody waits for the whole copy) and copies every tile that has reached its final version out

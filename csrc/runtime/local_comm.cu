@@ -305,7 +305,6 @@ int sar_local_run(sar_local_comm* c, const sar_program* prog, void* const* bufs,
       P.gate_rounds = gated ? 1u : 0u;
       P.gate_slack = sar::gate_slack(g.tiles_per_chunk);
       P.stages = stages > 0 ? (uint32_t)stages : (uint32_t)sar_table_stages_hint(t);
-      P.store_window = o->store_window > 0 ? (uint32_t)o->store_window : 0u;
       P.lane1_eighths = (uint32_t)sar_table_lane1_eighths(t);
       if (mc_alloc) {
         for (int grp = 0; grp < 2; ++grp) {

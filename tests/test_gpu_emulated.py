@@ -323,3 +323,44 @@ def test_scale_cast_edges(count, offset):
                 ops.scale_cast(src, src, 0.3)
                 torch.cuda.synchronize()
                 assert torch.equal(src, want)
+
+
+@pytest.mark.parametrize("stages", [2, 3, 6])
+@pytest.mark.parametrize("alg,blocks,tile_bytes", [("stragglar", 1, 2048), ("rsag", 2, 2048), ("stragglar_a2a", 3, 98304),
+                                                   ("ring", 1, 33280)])
+@pytest.mark.parametrize("staged", [False, True])
+def test_bulk_copy_ring(alg, blocks, tile_bytes, stages, staged):
+    """The hand-over between the roles of a block: rings from two stages up, many items a block (more than a storer's
+    queue holds), items of one piece, of several and with a ragged last one, copies that skip the adders, conversions."""
+    from stragglar_b200 import ops
+    n, count = 8, 150_003
+    comm = ops.LocalComm(n, emulate=True)
+    prog = sc.compile_program(alg, n)
+    xs = _inputs(n, count, torch.float32)
+    wire = torch.bfloat16 if staged else torch.float32
+    want = torch.stack([x.to(wire).double() for x in xs]).sum(0)
+    arena = [torch.zeros(count, dtype=wire, device="cuda:0") for _ in range(n)] if staged else xs
+    comm.run(prog, arena, path="tma", blocks=blocks, tile_bytes=tile_bytes, stages=stages, timeout_s=5.0,
+             user_tensors=xs if staged else None)
+    comm.sync()
+    for x in xs:
+        torch.testing.assert_close(x.double(), want, **TOL[wire])
+    comm.close()
+
+
+def test_wait_runs_out_on_the_bulk_copy_path():
+    """As above with the roles of the bulk-copy path: all of them leave, and the communicator works again."""
+    from stragglar_b200 import ops
+    n, count = 4, 100_000
+    comm = ops.LocalComm(n, emulate=True)
+    prog = sc.compile_program("stragglar", n)
+    comm.run(prog, _inputs(n, count, torch.float32), path="tma", blocks=2, tile_bytes=4096, delay_ms=[0, 0, 0, 400.0], timeout_s=0.05)
+    comm.sync(check=False)
+    assert 0 < comm.last_status < 0x1000
+    ys = _inputs(n, count, torch.float32)
+    want = torch.stack([y.double() for y in ys]).sum(0)
+    comm.run(prog, ys, path="tma", blocks=2, tile_bytes=4096)
+    comm.sync()
+    for y in ys:
+        torch.testing.assert_close(y.double(), want, **TOL[torch.float32])
+    comm.close()
