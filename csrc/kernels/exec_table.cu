@@ -45,8 +45,12 @@ __device__ __forceinline__ void load_rank_params(const SarEmulParams& E, int r, 
 }
 static_assert(sizeof(SarLaunchParams) % 4 == 0, "params are copied word by word");
 
-template <typename T>
-__global__ void __launch_bounds__(512, 1) sar_emul_simt_kernel(const __grid_constant__ SarEmulParams E, int blocks_per_rank) {
+// MAX_THREADS 256: three blocks per SM at 80 registers a thread (a few spilled words), 512: one.  A block is a serial
+// chain here too, so the third one pays: 8 ranks, rhd, 64 MiB fp16 409 -> 394 us (simta 421 -> 392), 4-rank ring, 40 MB
+// 119 -> 110 us, 6 ranks, 12 MB 67.7 -> 62.6 us, against two blocks at 128 registers.  Four blocks at 64 registers with
+// half the vectors in flight: level on simt, 5 % slower on simta.
+template <typename T, int MAX_THREADS>
+__global__ void __launch_bounds__(MAX_THREADS, MAX_THREADS == 256 ? 3 : 1) sar_emul_simt_kernel(const __grid_constant__ SarEmulParams E, int blocks_per_rank) {
   __shared__ SarLaunchParams P;
   load_rank_params(E, blockIdx.x / blocks_per_rank, P);
   if (!(P.participants >> P.rank & 1)) return;
@@ -54,7 +58,7 @@ __global__ void __launch_bounds__(512, 1) sar_emul_simt_kernel(const __grid_cons
 }
 
 template <typename T, int THREADS>
-__global__ void __launch_bounds__(THREADS, 512 / THREADS) sar_emul_simta_kernel(const __grid_constant__ SarEmulParams E, int blocks_per_rank) {
+__global__ void __launch_bounds__(THREADS, THREADS == 256 ? 3 : 1) sar_emul_simta_kernel(const __grid_constant__ SarEmulParams E, int blocks_per_rank) {
   __shared__ SarLaunchParams P;
   __shared__ simta::Shared S;
   load_rank_params(E, blockIdx.x / blocks_per_rank, P);
@@ -345,7 +349,8 @@ int sar_cuda_emulated_fit(int dtype, int path, int threads, int stages, int num_
       return threads == simta::kThreadsShared
                  ? (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sar_emul_simta_kernel<T, simta::kThreadsShared>, simta::kThreadsShared, 0)
                  : (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sar_emul_simta_kernel<T, simta::kThreads>, simta::kThreads, 0);
-    return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sar_emul_simt_kernel<T>, threads <= 0 ? 512 : threads, 0);
+    if (threads == 256) return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sar_emul_simt_kernel<T, 256>, 256, 0);
+    return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sar_emul_simt_kernel<T, 512>, threads <= 0 ? 512 : threads, 0);
   });
   return sms * per_sm;
 }
@@ -383,7 +388,8 @@ int sar_cuda_launch_emulated(const SarLaunchParams* params, int n, int path, int
                  ? (int)cudaLaunchCooperativeKernel((void*)sar_emul_simta_kernel<T, simta::kThreadsShared>, dim3(n * blocks_per_rank), dim3(simta::kThreadsShared), args, 0, st)
                  : (int)cudaLaunchCooperativeKernel((void*)sar_emul_simta_kernel<T, simta::kThreads>, dim3(n * blocks_per_rank), dim3(simta::kThreads), args, 0, st);
     if (threads <= 0) threads = 512;
-    return (int)cudaLaunchCooperativeKernel((void*)sar_emul_simt_kernel<T>, dim3(n * blocks_per_rank), dim3(threads), args, 0, st);
+    return (int)cudaLaunchCooperativeKernel(threads == 256 ? (void*)sar_emul_simt_kernel<T, 256> : (void*)sar_emul_simt_kernel<T, 512>,
+                                            dim3(n * blocks_per_rank), dim3(threads), args, 0, st);
   });
 }
 

@@ -1491,7 +1491,7 @@ __device__ void run_rank_tma(const SarLaunchParams& P, uint32_t block, uint32_t 
 // reductions over, and pushes to, a whole multicast group go through the switch.
 namespace simta {
 constexpr int kThreads = 512;
-constexpr int kThreadsShared = 256;   // ranks on one device: two blocks per SM (see run_rank_simta)
+constexpr int kThreadsShared = 256;   // ranks on one device: several blocks per SM (see run_rank_simta)
 constexpr int kSlots = 2;
 constexpr int kPendRing = 16;
 struct PendEntry { const SarOp* op; uint32_t fidx; };   // a finished item on its way to the signal thread
@@ -1513,9 +1513,10 @@ struct Shared {
 template <int WORKERS> __device__ __forceinline__ void worker_bar() { asm volatile("bar.sync 1, %0;" ::"n"(WORKERS) : "memory"); }
 }  // namespace simta
 
-// THREADS per block: all but the last two warps are workers.  A block moves one tile at a time; with 256 threads two
-// of them fit an SM (125 registers a thread) and one copies while the other turns over.  8 ranks on one device, rhd,
-// 64 MiB fp16: 504 us with one 512-thread block per SM, 443 us with two of 256 threads, 424 us with tiles of 256 KiB.
+// THREADS per block: all but the last two warps are workers.  A block moves one tile at a time; with 256 threads
+// several of them fit an SM and one copies while another turns over.  8 ranks on one device, rhd, 64 MiB fp16: 504 us
+// with one 512-thread block per SM, 443 us with two of 256 threads, 424 us with tiles of 256 KiB, 392 us with three
+// blocks.
 template <typename T, int THREADS>
 __device__ void run_rank_simta(const SarLaunchParams& P, uint32_t block, uint32_t nblocks, simta::Shared& S) {
   using namespace simta;

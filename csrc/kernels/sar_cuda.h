@@ -22,7 +22,7 @@ int sar_cuda_launch(const struct SarLaunchParams* p, int path, int blocks, int t
 // n ranks emulated on the current device by ONE cooperative launch: params
 // points to n SarLaunchParams in host memory (read during the call), which
 // differ in rank, table, status, trace, delay and the caller's tensors only;
-// rank r is run by blocks [r*blocks_per_rank, (r+1)*blocks_per_rank).  On the simta path threads is 256 (two blocks
+// rank r is run by blocks [r*blocks_per_rank, (r+1)*blocks_per_rank).  On the simta path threads is 256 (three blocks
 // per SM) or anything else (512).  Fails with
 // cudaErrorCooperativeLaunchTooLarge when the blocks cannot all be resident.
 int sar_cuda_launch_emulated(const struct SarLaunchParams* params, int n, int path, int blocks_per_rank, int threads,

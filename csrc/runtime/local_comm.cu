@@ -115,9 +115,10 @@ static DevTable* upload(Rank& rk, const sar_table* t, int rank, char* err, int e
 // Launch shape of a collective whose ranks share one device: as many blocks per rank as can be resident together,
 // but no more than one per 16 KiB of a rank's buffer (tiles start at 2 KiB: below that the blocks find no work and
 // only lengthen the entry).  Every block is a serial chain of wait, move, announce, so bandwidth comes from their
-// number.  On the simt path 256 threads a block let two chains share an SM where 512 leave it one.
+// number.  On the simt path 256 threads a block let three chains share an SM where 512 leave it one.
 // 8 ranks, fp32, against 4 blocks per rank: 25 MiB 742 -> 199 us, 256 MiB 7.68 -> 1.61 ms (one bulk-copy block per SM;
-// two since then, see tma::Shared); 6 ranks, simt, 12 MB 349 -> 70 us (76 us with 512 threads a block).
+// two since then, see tma::Shared); 6 ranks, simt, 12 MB 349 -> 70 us (two blocks per SM;
+// 76 us with one of 512 threads).
 static int emulated_blocks(sar_local_comm* c, const sar_program* prog, int dtype, int path, int* threads, int stages, uint64_t bytes) {
   if (path == SAR_PATH_SIMTA || (path == SAR_PATH_SIMT && *threads <= 0)) *threads = 256;
   cudaSetDevice(c->ranks[0].dev);   // occupancy is that of the current device
