@@ -324,12 +324,13 @@ void ProcessGroupStragglar::run_program(Side& s, const sar::Program& prog, size_
     if (!(c.participants >> me & 1)) continue;
     int blocks = t.cuda() ? (opts_.blocks > 0 ? opts_.blocks : sar_cuda_pick_blocks(opts_.path, count * esize)) : 1;
     if (t.cuda() && opts_.blocks <= 0 && c.blocks_hint > 0 && c.blocks_hint < blocks) blocks = c.blocks_hint;
-    uint32_t stages = (uint32_t)c.stages_hint;
-    if (t.cuda() && opts_.blocks <= 0 && n == 1) { stages = 0; blocks = sar_cuda_lone_blocks(opts_.path, count * esize, &stages); }
+    if (t.cuda() && opts_.blocks <= 0 && n == 1) blocks = sar_cuda_lone_blocks(count * esize);
     const bool gated = c.gate_rounds && count * esize >= sar::gate_min_bytes();
     // staged launches poll a flag over the link for every tile they read from a peer, version 0 included: larger tiles
     const uint32_t tile_max = opts_.tile_bytes ? opts_.tile_bytes
-                            : (t.cuda() ? ((gated || (user && n > 1)) ? sar::gate_tile_bytes() : sar_cuda_default_tile_bytes(opts_.path)) : (128u << 10));
+                            : !t.cuda() ? (128u << 10)
+                            : n == 1 ? sar_cuda_lone_tile_bytes(opts_.path)
+                            : (gated || user) ? sar::gate_tile_bytes() : sar_cuda_default_tile_bytes(opts_.path);
     const uint32_t tile_elems = sar::pick_tile_elems(count, esize, (uint32_t)c.num_chunks, (uint32_t)blocks, 2048, tile_max);
     const SarGeom g = sar::make_geom(count, esize, (uint32_t)c.num_chunks, tile_elems);
     TORCH_CHECK((uint64_t)g.tiles_per_chunk * g.num_chunks <= SAR_FLAG_CAPACITY, "tensor too large for the flag array");
@@ -370,7 +371,7 @@ void ProcessGroupStragglar::run_program(Side& s, const sar::Program& prog, size_
       }
       P.gate_rounds = gated ? 1u : 0u;
       P.gate_base = epoch64; P.gate_slack = sar::gate_slack(g.tiles_per_chunk);
-      P.stages = stages;
+      P.stages = n == 1 ? 0u : (uint32_t)c.stages_hint;
       P.lane1_eighths = (uint32_t)c.lane1_eighths;
       int launch_blocks = blocks;
       if (user && n == 1) {

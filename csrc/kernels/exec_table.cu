@@ -295,15 +295,11 @@ int sar_cuda_pick_blocks(int path, uint64_t bytes) {
   (void)path;
   return (int)(b < (uint64_t)lo ? lo : (b > (uint64_t)hi ? hi : b));
 }
-int sar_cuda_lone_blocks(int path, uint64_t bytes, uint32_t* stages) {
-  uint64_t full = 148;
-  if (path == SAR_PATH_TMA) {
-    if (*stages == 0) *stages = 3;
-    if (*stages <= 3) full = 296;
-  }
+int sar_cuda_lone_blocks(uint64_t bytes) {
   const uint64_t b = (bytes + (32u << 10) - 1) / (32u << 10);
-  return (int)(b < 32 ? 32 : (b > full ? full : b));
+  return (int)(b < 32 ? 32 : (b > 148 ? 148 : b));
 }
+uint32_t sar_cuda_lone_tile_bytes(int path) { return path == SAR_PATH_TMA ? (uint32_t)tma::kStageBytes : sar_cuda_default_tile_bytes(path); }
 uint32_t sar_cuda_default_tile_bytes(int path) { return path == SAR_PATH_TMA ? (64u << 10) : (128u << 10); }
 
 int sar_cuda_launch(const SarLaunchParams* params, int path, int blocks, int threads, void* stream) {
@@ -315,9 +311,8 @@ int sar_cuda_launch(const SarLaunchParams* params, int path, int blocks, int thr
   return with_dtype(p->dtype, [&](auto tag) -> int {
     using T = decltype(tag);
     if (path == SAR_PATH_TMA) {
-      // The whole ring: ranks on devices of their own have an SM to themselves.  A lone rank streams its own memory and
-      // takes what it asks for, two blocks per SM with three stages (sar_cuda_lone_blocks).
-      const uint32_t smem = tma::smem_bytes(table_ops(*p), p->nranks == 1 ? tma::stages_in_use(p->stages) : (uint32_t)tma::kStages);
+      // the whole ring: ranks on devices of their own have an SM to themselves
+      const uint32_t smem = tma::smem_bytes(table_ops(*p), (uint32_t)tma::kStages);
       int e = allow_smem(sar_exec_tma_kernel<T>, smem);
       if (e) return e;
       sar_exec_tma_kernel<T><<<blocks, tma::kThreads, smem, st>>>(*p);

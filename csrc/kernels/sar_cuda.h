@@ -31,11 +31,12 @@ int sar_cuda_default_blocks(int path);
 // blocks per rank for a buffer of `bytes`: few for small messages (latency bound, and the SMs
 // are left to the compute that overlaps the collective), up to 128 for large ones
 int sar_cuda_pick_blocks(int path, uint64_t bytes);
-// Blocks of a lone rank (a group of one: the collective scales the rank's own memory, and no link or peer bounds it):
-// one per ring stage's worth of data (32 KiB) up to one per SM or, on the bulk-copy path unless the caller has chosen
-// more ring stages, two per SM with three stages each (1 GiB fp32: 381 us with one block of six stages per SM, 356 us
-// with two; three blocks or smaller stages 356 to 388 us).  *stages (0: free choice) is set to match.
-int sar_cuda_lone_blocks(int path, uint64_t bytes, uint32_t* stages);
+// Launch shape of a lone rank (a group of one: the collective scales the rank's own memory, and no link or peer bounds
+// it): a block per ring stage's worth of data (32 KiB) up to one per SM, and on the bulk-copy path tiles of one stage, so
+// that consecutive pieces go to different storers.  1 GiB fp32: 338 us (6.35 TB/s); with tiles of 64 KiB 357 us, with
+// two blocks of three stages per SM 349 us (64 KiB tiles: 354 us).
+int sar_cuda_lone_blocks(uint64_t bytes);
+uint32_t sar_cuda_lone_tile_bytes(int path);
 uint32_t sar_cuda_default_tile_bytes(int path);
 int sar_cuda_max_emulated_blocks(int dtype, int path, int threads);   // resident blocks on the current device
 // the same for a launch of 256-thread blocks on the simta path (threads = 256), or with `stages` ring stages (0: all; bulk-copy path) and tables of at most num_ops ops

@@ -234,16 +234,13 @@ int sar_local_run(sar_local_comm* c, const sar_program* prog, void* const* bufs,
     if (path == SAR_PATH_TMA && stages <= 0) stages = 3;   // two blocks per SM (see emulated_blocks)
     blocks = emulated_blocks(c, prog, dtype, path, &threads, stages, count * esize);
   }
-  if (n == 1 && !c->emulate && o->blocks <= 0) {
-    uint32_t st = stages > 0 ? (uint32_t)stages : 0u;
-    blocks = sar_cuda_lone_blocks(path, count * esize, &st);
-    stages = (int)st;
-  }
+  const bool lone = n == 1 && !c->emulate && o->blocks <= 0;
+  if (lone) { blocks = sar_cuda_lone_blocks(count * esize); if (stages <= 0) stages = 6; }
   const double timeout_s = o->timeout_s > 0 ? o->timeout_s : 10.0;
   // Emulated ranks, simt and simta: tiles of up to 256 KiB, because the wait, the block barriers and the fence around
   // a tile are not hidden behind another one (ring, 4 ranks, 40 MB: 124 us against 137 with 128 KiB; level where the
   // blocks outnumber the tiles).  The bulk-copy ring hides them: 64 KiB.
-  const uint32_t tile_max = o->tile_bytes ? o->tile_bytes
+  const uint32_t tile_max = o->tile_bytes ? o->tile_bytes : lone ? sar_cuda_lone_tile_bytes(path)
                           : (c->emulate && path != SAR_PATH_TMA ? (256u << 10) : sar_cuda_default_tile_bytes(path));
   std::vector<bool> delayed(n, false);
 
