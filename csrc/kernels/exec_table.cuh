@@ -650,9 +650,43 @@ __device__ __forceinline__ void store_from_float(void* base, uint64_t e, int dty
   else { __half b = __float2half_rn(v); h = *reinterpret_cast<unsigned short*>(&b); }
   ((unsigned short*)base)[e] = h;
 }
+// N elements (one wire vector's worth) of the caller's tensor as floats, and back, with vector accesses: 32 bytes of fp32
+// or 16 of a 2-byte type next to a 2-byte wire, 8 bytes of a 2-byte type next to an fp32 wire.  `p` is aligned to that
+// (to 16 bytes for the 32).
+template <int N> __device__ __forceinline__ void load_user_vec(const char* p, int dtype, float* f) {
+  if (dtype == SAR_F32) {
+#pragma unroll
+    for (int h = 0; h < N / 4; ++h) Vec<float>::unpack(ld_vec_sys(p + 16 * h), f + 4 * h);
+    return;
+  }
+  uint4 v = make_uint4(0, 0, 0, 0);
+  if constexpr (N == 8) v = ld_vec_sys(p);
+  else asm volatile("ld.relaxed.sys.global.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p) : "memory");
+  float t[8];
+  if (dtype == SAR_BF16) Vec<__nv_bfloat16>::unpack(v, t);
+  else Vec<__half>::unpack(v, t);
+#pragma unroll
+  for (int i = 0; i < N; ++i) f[i] = t[i];
+}
+template <int N> __device__ __forceinline__ void store_user_vec(char* p, int dtype, const float* f) {
+  if (dtype == SAR_F32) {
+#pragma unroll
+    for (int h = 0; h < N / 4; ++h) st_vec(p + 16 * h, Vec<float>::pack(f + 4 * h));
+    return;
+  }
+  float t[8] = {};
+#pragma unroll
+  for (int i = 0; i < N; ++i) t[i] = f[i];
+  const uint4 v = dtype == SAR_BF16 ? Vec<__nv_bfloat16>::pack(t) : Vec<__half>::pack(t);
+  if constexpr (N == 8) st_vec(p, v);
+  else asm volatile("st.global.v2.u32 [%0], {%1,%2};" ::"l"(p), "r"(v.x), "r"(v.y) : "memory");
+}
+
 // A staging tile: SAR_STAGE_IN copies the caller's elements into the own slot (wire type T), SAR_STAGE_OUT copies
 // the own slot into the caller's output.  Same element type and 16-byte aligned on both sides: vector copies;
-// otherwise the elements are converted one wire vector at a time.  `tid` of `nth` threads work together.
+// otherwise the elements are converted one wire vector at a time, with vector accesses on both sides where the caller's
+// side is aligned (8 ranks, 25 MiB fp32 buckets, bf16 wire, simt: 317 -> 203 us; element by element before).  `tid` of
+// `nth` threads work together.
 template <typename T>
 __device__ void stage_tile(const SarLaunchParams& P, const Item& it, const uint32_t tid, const uint32_t nth) {
   constexpr int N = Vec<T>::N;
@@ -684,7 +718,27 @@ __device__ void stage_tile(const SarLaunchParams& P, const Item& it, const uint3
   const void* src = in ? P.user_in : (const void*)own;
   void* dst = in ? (void*)own : P.user_out;
   const int sdt = in ? udt : P.dtype, ddt = in ? P.dtype : udt;
-  for (uint32_t v = tid; v < nvec; v += nth) {
+  uint32_t v = tid;
+  const uint32_t usz = udt == SAR_F32 ? 4u : 2u;
+  char* const user = (in ? (char*)const_cast<void*>(P.user_in) : (char*)P.user_out) + it.elem0 * usz;
+  if (((uintptr_t)user & 15) == 0) {
+    char* const slot = own + it.elem0 * sizeof(T);
+    const uint32_t ub = N * usz;
+    for (; v + nth < nvec; v += 2 * nth) {
+      float f[2][N];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        if (in) load_user_vec<N>(user + (size_t)(v + u * nth) * ub, udt, f[u]);
+        else Vec<T>::unpack(ld_vec_sys(slot + (size_t)(v + u * nth) * 16), f[u]);
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        if (in) st_vec(slot + (size_t)(v + u * nth) * 16, Vec<T>::pack(f[u]));
+        else store_user_vec<N>(user + (size_t)(v + u * nth) * ub, udt, f[u]);
+      }
+    }
+  }
+  for (; v < nvec; v += nth) {
     float f[N];
 #pragma unroll
     for (int i = 0; i < N; ++i) f[i] = load_as_float(src, it.elem0 + (uint64_t)v * N + i, sdt);
