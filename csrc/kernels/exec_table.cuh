@@ -1221,11 +1221,16 @@ __device__ void convert_piece(unsigned char* dst, int ddt, const unsigned char* 
     if (ddt == SAR_BF16) convert_pair<NT, SAR_F32, SAR_BF16>(dst, src, elems, tid);
     else convert_pair<NT, SAR_F32, SAR_F16>(dst, src, elems, tid);
   } else if (sdt == SAR_BF16) {
-    convert_pair<NT, SAR_BF16, SAR_F32>(dst, src, elems, tid);
+    if (ddt == SAR_F32) convert_pair<NT, SAR_BF16, SAR_F32>(dst, src, elems, tid);
+    else convert_pair<NT, SAR_BF16, SAR_F16>(dst, src, elems, tid);
   } else {
-    convert_pair<NT, SAR_F16, SAR_F32>(dst, src, elems, tid);
+    if (ddt == SAR_F32) convert_pair<NT, SAR_F16, SAR_F32>(dst, src, elems, tid);
+    else convert_pair<NT, SAR_F16, SAR_BF16>(dst, src, elems, tid);
   }
 }
+// Whether a staged piece is converted (into the second half of its stage) on its way between the caller's tensor and
+// the slot.  The types decide, not the sizes: fp16 and bf16 are two bytes each.
+__device__ __forceinline__ bool staging_converts(const SarLaunchParams& P) { return P.user_dtype != P.dtype; }
 
 // Roles of a block (256 threads):
 //   warp 0, one thread     producer: walks the items, waits for their operands
@@ -1315,7 +1320,7 @@ __device__ void run_rank_tma(const SarLaunchParams& P, uint32_t block, uint32_t 
           }
           // pieces of whole 16-byte vectors on both sides (8 elements); a converted piece uses half a stage per side
           const uint32_t big = ssz > dsz ? ssz : dsz;
-          const uint32_t piece = sdt == ddt ? (uint32_t)kStageBytes / ssz : (uint32_t)(kStageBytes / 2) / big;
+          const uint32_t piece = !staging_converts(P) ? (uint32_t)kStageBytes / ssz : (uint32_t)(kStageBytes / 2) / big;
           const uint32_t body = it.nelem & ~7u, tail = it.nelem & 7u;
           uint32_t done = 0;
           do {
@@ -1410,7 +1415,7 @@ __device__ void run_rank_tma(const SarLaunchParams& P, uint32_t block, uint32_t 
           Item sit{};
           sit.op = op; sit.elem0 = d.item_elem0; sit.nelem = d.item_elems;
           stage_tile<T>(P, sit, ctid, CT);
-        } else if (d.bytes != d.dst_bytes) {
+        } else if (staging_converts(P)) {
           // convert the piece from the first half of the stage into the second
           const bool in = op->kind == SAR_STAGE_IN;
           const int sdt = in ? P.user_dtype : P.dtype, ddt = in ? P.dtype : P.user_dtype;
@@ -1482,7 +1487,7 @@ __device__ void run_rank_tma(const SarLaunchParams& P, uint32_t block, uint32_t 
       if (op->kind >= SAR_STAGE_IN) {
         if (d.dst_bytes) {
           char* dst = op->kind == SAR_STAGE_IN ? (char*)P.comm.buf[P.rank] : (char*)P.user_out;
-          bulk_store(dst + d.dst_off, d.bytes != d.dst_bytes ? stage + kStageBytes / 2 : stage, d.dst_bytes);
+          bulk_store(dst + d.dst_off, staging_converts(P) ? stage + kStageBytes / 2 : stage, d.dst_bytes);
         }
       } else if (d.bytes) {
         if (op->kind != SAR_PUSH) bulk_store((char*)P.comm.buf[P.rank] + d.byte_off, stage, d.bytes);

@@ -116,6 +116,29 @@ def test_lone_rank_of_every_size():
     run_ranks(1, _lone_rank)
 
 
+def _two_byte_wire(rank, world):
+    import stragglar_b200.parallel as sp
+    torch.cuda.set_device(rank)
+    dev = torch.device("cuda", rank)
+    for count in (3, 8 * 1024 + 1, 1 << 20):
+        x = torch.empty(count, device=dev).normal_(generator=torch.Generator(device=dev).manual_seed(count))
+        x[0], x[1], x[2] = 3e4, -1e6, 1e-6       # near and beyond the range of fp16, and one of its subnormal numbers
+        for dtype, wire in ((torch.float16, torch.bfloat16), (torch.bfloat16, torch.float16)):
+            t = x.to(dtype)
+            want = t.to(wire).to(dtype)          # the mean of one rank, rounded once to the wire
+            assert not torch.equal(t, want)
+            sp.all_reduce_ex(t, average=True, comm_dtype=wire).wait()
+            assert torch.equal(t, want), (count, dtype, wire)
+    torch.cuda.synchronize()
+    assert sp.check_status(dev) == 0 and sp.check_guards(dev)
+
+
+def test_two_byte_wire_types_are_converted():
+    """all_reduce_ex of an fp16 tensor over a bf16 wire, and the reverse: the elements have the same size, not the same
+    meaning."""
+    run_ranks(1, _two_byte_wire)
+
+
 @pytest.mark.multigpu
 def test_backend_on_all_gpus():
     world = min(torch.cuda.device_count(), 8)

@@ -364,3 +364,29 @@ def test_wait_runs_out_on_the_bulk_copy_path():
     for y in ys:
         torch.testing.assert_close(y.double(), want, **TOL[torch.float32])
     comm.close()
+
+
+@pytest.mark.parametrize("path", PATHS)
+@pytest.mark.parametrize("wire,user", [(torch.bfloat16, torch.float16), (torch.float16, torch.bfloat16)])
+@pytest.mark.parametrize("offset", [0, 1])   # elements: bulk copies or vectors, and element by element
+@pytest.mark.parametrize("shape", [{}, {"blocks": 3, "tile_bytes": 4096}])
+def test_staged_mode_between_the_two_byte_types(wire, user, path, offset, shape):
+    """fp16 and bf16 have the same size and are not the same: both ways of a staged collective convert."""
+    from stragglar_b200 import ops
+    n, count = 4, 70_005
+    comm = ops.LocalComm(n, emulate=True)
+    prog = sc.compile_program("rsag", n)
+    users = []
+    for x in _inputs(n, count, torch.float32):
+        u = torch.empty(count + offset, dtype=user, device="cuda:0")[offset:]
+        u.copy_(x)
+        users.append(u)
+    want = torch.stack([u.to(wire).double() for u in users]).sum(0) * 0.5
+    arena = [torch.full((count,), float("nan"), dtype=wire, device="cuda:0") for _ in range(n)]
+    comm.run(prog, arena, path=path, scale=0.5, timeout_s=5.0, user_tensors=users, **shape)
+    comm.sync()
+    # one rounding to each type, half an ulp each (2^-8 for 8 significant bits in bf16, 2^-11 for 11 in fp16), after a sum
+    # of four values below 1 in fp32
+    for u in users:
+        torch.testing.assert_close(u.double(), want, rtol=2 ** -8 + 2 ** -11 + 2 ** -18, atol=1e-6)
+    comm.close()
