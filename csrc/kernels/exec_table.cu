@@ -280,8 +280,13 @@ int grid_for(uint64_t count, int threads) {
   uint64_t b = (count + threads - 1) / threads;
   return (int)(b < 1 ? 1 : (b > 148 * 16 ? 148 * 16 : b));
 }
-template <typename K> int allow_smem(K kernel, size_t bytes) {
-  return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+// Lets a bulk-copy kernel take the largest ring and table.  The limit is state of the kernel on the device, shared by
+// every thread of the process: it is always set to the same value, never to what one launch needs, or a thread could
+// lower it between another one's call and its launch.  A launch occupies what it asks for, whatever the limit.
+template <typename K> int allow_smem(K kernel) {
+  constexpr uint32_t kMost = tma::smem_bytes(SAR_MAX_OPS, (uint32_t)tma::kStages);
+  static_assert(kMost <= 227u << 10, "a block may have 227 KB of shared memory");
+  return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMost);
 }
 }  // namespace
 
@@ -313,7 +318,7 @@ int sar_cuda_launch(const SarLaunchParams* params, int path, int blocks, int thr
     if (path == SAR_PATH_TMA) {
       // the whole ring: ranks on devices of their own have an SM to themselves
       const uint32_t smem = tma::smem_bytes(table_ops(*p), (uint32_t)tma::kStages);
-      int e = allow_smem(sar_exec_tma_kernel<T>, smem);
+      int e = allow_smem(sar_exec_tma_kernel<T>);
       if (e) return e;
       sar_exec_tma_kernel<T><<<blocks, tma::kThreads, smem, st>>>(*p);
     } else if (path == SAR_PATH_SIMTA) {
@@ -337,7 +342,7 @@ int sar_cuda_emulated_fit(int dtype, int path, int threads, int stages, int num_
     using T = decltype(tag);
     if (path == SAR_PATH_TMA) {
       const uint32_t smem = tma::smem_bytes((uint32_t)num_ops, tma::stages_in_use((uint32_t)stages));
-      allow_smem(sar_emul_tma_kernel<T>, smem);
+      allow_smem(sar_emul_tma_kernel<T>);
       return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sar_emul_tma_kernel<T>, tma::kThreads, smem);
     }
     if (path == SAR_PATH_SIMTA)
@@ -373,7 +378,7 @@ int sar_cuda_launch_emulated(const SarLaunchParams* params, int n, int path, int
       uint32_t nops = 0;
       for (int r = 0; r < n; ++r) nops = table_ops(params[r]) > nops ? table_ops(params[r]) : nops;
       const uint32_t smem = tma::smem_bytes(nops, tma::stages_in_use(E.common.stages));
-      int e = allow_smem(sar_emul_tma_kernel<T>, smem);
+      int e = allow_smem(sar_emul_tma_kernel<T>);
       if (e) return e;
       return (int)cudaLaunchCooperativeKernel((void*)sar_emul_tma_kernel<T>, dim3(n * blocks_per_rank), dim3(tma::kThreads),
                                               args, smem, st);

@@ -1092,11 +1092,11 @@ struct Shared {
 
 // ring stages in use: fewer stages keep fewer bytes in flight per block
 __host__ __device__ __forceinline__ uint32_t stages_in_use(uint32_t asked) { return (asked >= 2 && asked < (uint32_t)kStages) ? asked : (uint32_t)kStages; }
-__host__ __device__ __forceinline__ uint32_t ops_offset() { return (uint32_t)((sizeof(Shared) + 15) / 16 * 16); }
-__host__ __device__ __forceinline__ uint32_t ring_offset(uint32_t nops) {
+__host__ __device__ __forceinline__ constexpr uint32_t ops_offset() { return (uint32_t)((sizeof(Shared) + 15) / 16 * 16); }
+__host__ __device__ __forceinline__ constexpr uint32_t ring_offset(uint32_t nops) {
   return (uint32_t)((ops_offset() + nops * (sizeof(OpGeom) + sizeof(SarOp)) + 127) / 128 * 128);
 }
-__host__ __device__ __forceinline__ uint32_t smem_bytes(uint32_t nops, uint32_t stages) { return ring_offset(nops) + stages * (uint32_t)kStageBytes; }
+__host__ __device__ __forceinline__ constexpr uint32_t smem_bytes(uint32_t nops, uint32_t stages) { return ring_offset(nops) + stages * (uint32_t)kStageBytes; }
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void mbar_init(uint64_t* b, uint32_t count) {

@@ -2,6 +2,7 @@
 cooperative launch), against a plain PyTorch fp32/fp64 reference.  Both data
 paths (simt loads/stores and the bulk-copy pipeline) run the same tables."""
 import os
+import threading
 
 import pytest
 import torch
@@ -389,4 +390,34 @@ def test_staged_mode_between_the_two_byte_types(wire, user, path, offset, shape)
     # of four values below 1 in fp32
     for u in users:
         torch.testing.assert_close(u.double(), want, rtol=2 ** -8 + 2 ** -11 + 2 ** -18, atol=1e-6)
+    comm.close()
+
+
+def test_launches_beside_another_threads_smaller_ring():
+    """The shared-memory limit of a kernel belongs to the device, not to a call: a thread that asks for a launch with few
+    ring stages leaves the launches of another thread, with the whole ring, alone."""
+    from stragglar_b200 import ops
+    n, count = 2, 1000
+    comm = ops.LocalComm(n, emulate=True)
+    prog = sc.compile_program("rsag", n)
+    xs = _inputs(n, count, torch.float32)
+    want = torch.stack([x.double() for x in xs]).mean(0)
+    stop = threading.Event()
+
+    def ask():
+        while not stop.is_set():
+            ops.cuda_lib().sar_cuda_emulated_fit(0, ops.local.PATHS["tma"], 0, 2, 1)
+
+    other = threading.Thread(target=ask)
+    other.start()
+    try:
+        for _ in range(50):
+            for _ in range(40):
+                comm.run(prog, xs, path="tma", blocks=1, stages=6, scale=0.5, timeout_s=5.0)
+            comm.sync()
+    finally:
+        stop.set()
+        other.join()
+    for x in xs:
+        torch.testing.assert_close(x.double(), want, **TOL[torch.float32])
     comm.close()
