@@ -68,6 +68,7 @@ void sar_table_final_ver(const sar_table* t, int rank, uint8_t* out) {
   for (size_t c = 0; c < fv.size() && c < SAR_MAX_CHUNKS; ++c) out[c] = fv[c];
 }
 int sar_table_gate_rounds(const sar_table* t) { return t->c.gate_rounds ? 1 : 0; }
+int sar_table_gate_asked(const sar_table* t) { return t->c.gate_asked ? 1 : 0; }
 uint64_t sar_gate_min_bytes(void) { return sar::gate_min_bytes(); }
 int sar_table_lane1_eighths(const sar_table* t) { return t->c.lane1_eighths; }
 int sar_table_validate(const sar_table* t, int rank, int nranks, char* err, int errlen) {

@@ -30,6 +30,7 @@ int sar_program_num_phases(const sar_program* p);
 const sar_table* sar_program_phase(const sar_program* p, int i);
 int sar_table_channel(const sar_table* t);
 int sar_table_gate_rounds(const sar_table* t);   // 1: launch with round gating (for buffers of sar_gate_min_bytes() or more)
+int sar_table_gate_asked(const sar_table* t);    // 1: gated because STRAGGLAR_GATE asked for it when the program was compiled
 uint64_t sar_gate_min_bytes(void);
 // 0 when rank's table is well-formed for a communicator of nranks (see validate_rank_table); else 1 and the reason
 int sar_table_validate(const sar_table* t, int rank, int nranks, char* err, int errlen);

@@ -368,7 +368,10 @@ Plan plan_by_name(const std::string& alg, int n, bool prephase, const Schedule* 
   // STRAGGLAR_GATE=0 switches it off, STRAGGLAR_GATE=all gates every algorithm.
   p.gate_rounds = alg == "stragglar" && n >= 4;
   const char* gate = getenv("STRAGGLAR_GATE");
-  if (gate && *gate) p.gate_rounds = !strcmp(gate, "all") || (atoi(gate) != 0 && alg == "stragglar" && n >= 4);
+  if (gate && *gate) {
+    p.gate_rounds = !strcmp(gate, "all") || (atoi(gate) != 0 && alg == "stragglar" && n >= 4);
+    p.gate_asked = p.gate_rounds;
+  }
   // share of the blocks given to the forwarding lane (eighths); half unless STRAGGLAR_LANE1_EIGHTHS says otherwise
   // (forwarding moves n-2 chunks per chunk matched: the model of the executor prefers 5/8 at 32 blocks)
   const char* l1 = getenv("STRAGGLAR_LANE1_EIGHTHS");
@@ -610,6 +613,7 @@ Compiled compile(const Plan& plan, const std::vector<int>& l2p_in, int n_physica
   for (const RankTable& rt : out.ranks)
     for (const SarOp& op : rt.ops)
       if (op.round >= SAR_GATE_ALL_DONE) out.gate_rounds = false;   // does not fit the announcement word
+  out.gate_asked = plan.gate_asked && out.gate_rounds;
   // result check
   const uint32_t want = full_mask(n);
   for (int r : plan.participants) {

@@ -68,6 +68,7 @@ struct Plan {
   int blocks_hint = 0;            // largest block count per rank worth using (0: no preference)
   int stages_hint = 0;            // bulk-copy path: ring stages per block this plan runs best with (0: all)
   bool gate_rounds = false;       // run the rounds one after the other (see SAR_GATE_ALL_DONE in table.h)
+  bool gate_asked = false;        // ... because STRAGGLAR_GATE asked for it, not by default
   int lane1_eighths = 4;          // two lanes: share of the blocks that forwarding (lane 1) gets, in eighths
   bool two_lanes = false;         // forwarding ops go to lane 1 (their own blocks), the rest to lane 0
   bool split_copies = false;      // forward a chunk as two half-chunk ops, interleaved tile by tile, so that
@@ -110,6 +111,7 @@ struct Compiled {
   int blocks_hint = 0;    // upper bound of the blocks per rank this table runs best with (0: none)
   int stages_hint = 0;    // bulk-copy path: ring stages per block (0: all); fewer stages keep fewer bytes in flight
   bool gate_rounds = false;   // launch with round gating (every rank of a launch must agree)
+  bool gate_asked = false;    // gated on request (STRAGGLAR_GATE when the program was compiled), not by default
   int lane1_eighths = 4;      // share of the blocks of lane 1, in eighths (see sar_lane_of_block)
   std::vector<RankTable> ranks;          // by physical rank
   std::vector<int> logical_to_physical;

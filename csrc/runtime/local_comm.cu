@@ -4,7 +4,6 @@
 
 #include <algorithm>
 #include <cstdio>
-#include <cstdlib>
 #include <cstring>
 #include <map>
 #include <string>
@@ -269,9 +268,8 @@ int sar_local_run(sar_local_comm* c, const sar_program* prog, void* const* bufs,
     if (o->blocks <= 0 && !c->emulate && hint > 0 && hint < pblocks) pblocks = hint;
     // Gating keeps the rounds of a matching-based schedule from contending for the ports of the switch.  Emulated
     // ranks have no ports, only the hand-shake's cost (256 MiB, 8 ranks: 1140 us gated, 1048 us free-running): they
-    // are gated when STRAGGLAR_GATE asks for it.
-    const char* gate_env = getenv("STRAGGLAR_GATE");
-    const bool gate_wanted = !c->emulate || (gate_env && *gate_env);
+    // are gated when that was asked for (STRAGGLAR_GATE, read when the program is compiled).
+    const bool gate_wanted = !c->emulate || sar_table_gate_asked(t);
     const bool gated = gate_wanted && sar_table_gate_rounds(t) && count * esize >= sar_gate_min_bytes();
     const uint32_t ptile_max = (gated && !o->tile_bytes && !c->emulate) ? sar::gate_tile_bytes() : tile_max;
     const uint32_t tile_elems = sar_pick_tile_elems(count, esize, nch, (uint32_t)pblocks, 2048, ptile_max);

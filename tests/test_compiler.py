@@ -256,6 +256,18 @@ def test_round_gating_attribute_and_host_execution(monkeypatch):
     assert not sc.compile_program("stragglar", 8).main.gate_rounds
 
 
+def test_round_gating_on_request_is_part_of_the_program(monkeypatch):
+    """Whether gating was asked for is settled when a program is compiled, like gating itself."""
+    monkeypatch.delenv("STRAGGLAR_GATE", raising=False)
+    by_default = sc.compile_program("stragglar", 8)
+    assert by_default.main.gate_rounds and not by_default.main.gate_asked
+    for value, alg, asked in (("1", "stragglar", True), ("1", "ring", False), ("all", "ring", True), ("0", "stragglar", False)):
+        monkeypatch.setenv("STRAGGLAR_GATE", value)
+        prog = sc.compile_program(alg, 8)
+        assert prog.main.gate_asked == asked and prog.main.gate_rounds == asked, (value, alg)
+        assert not by_default.main.gate_asked
+
+
 def test_lane_split_share(monkeypatch):
     """STRAGGLAR_LANE1_EIGHTHS moves blocks between the two lanes: every split runs to the same sums and the
     default (half, alternating) is unchanged."""

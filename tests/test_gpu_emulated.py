@@ -421,3 +421,26 @@ def test_launches_beside_another_threads_smaller_ring():
     for x in xs:
         torch.testing.assert_close(x.double(), want, **TOL[torch.float32])
     comm.close()
+
+
+def test_gating_is_decided_when_the_program_is_compiled(monkeypatch):
+    """A program that was compiled with STRAGGLAR_GATE keeps its rounds apart when the variable is gone at run time."""
+    from stragglar_b200 import ops
+    n = 8
+    monkeypatch.setenv("STRAGGLAR_GATE_SLACK", "0")
+    monkeypatch.setenv("STRAGGLAR_GATE_MIN_BYTES", "0")
+    monkeypatch.setenv("STRAGGLAR_GATE", "1")
+    prog = sc.compile_program("stragglar", n)
+    monkeypatch.delenv("STRAGGLAR_GATE")
+    comm = ops.LocalComm(n, emulate=True)
+    xs = _inputs(n, 50_003, torch.float32)
+    want = torch.stack([x.double() for x in xs]).sum(0)
+    comm.run(prog, xs, path="tma", blocks=2, tile_bytes=4096, timeout_s=5.0, trace_rounds=True)
+    comm.sync()
+    for x in xs:
+        torch.testing.assert_close(x.double(), want, **TOL[torch.float32])
+    tr = comm.round_trace()
+    rounds = sorted({k for t in tr for k in t})
+    for a, b in zip(rounds, rounds[1:]):
+        assert max(t[a][1] for t in tr if a in t) <= min(t[b][0] for t in tr if b in t)
+    comm.close()
