@@ -11,7 +11,7 @@ extern __shared__ __align__(128) unsigned char sar_smem[];
 
 template <typename T>
 __global__ void __launch_bounds__(512, 1) sar_exec_simt_kernel(const __grid_constant__ SarLaunchParams P) {
-  run_rank_simt<T>(P, blockIdx.x, gridDim.x);
+  run_rank_simt<T>(P, blockIdx.x, gridDim.x, sar_smem);
 }
 
 template <typename T>
@@ -54,7 +54,7 @@ __global__ void __launch_bounds__(MAX_THREADS, MAX_THREADS == 256 ? 3 : 1) sar_e
   __shared__ SarLaunchParams P;
   load_rank_params(E, blockIdx.x / blocks_per_rank, P);
   if (!(P.participants >> P.rank & 1)) return;
-  run_rank_simt<T>(P, blockIdx.x % blocks_per_rank, blocks_per_rank);
+  run_rank_simt<T>(P, blockIdx.x % blocks_per_rank, blocks_per_rank, sar_smem);
 }
 
 template <typename T, int THREADS>
@@ -325,7 +325,7 @@ int sar_cuda_launch(const SarLaunchParams* params, int path, int blocks, int thr
       sar_exec_simta_kernel<T><<<blocks, simta::kThreads, 0, st>>>(*p);
     } else {
       if (threads <= 0) threads = 512;
-      sar_exec_simt_kernel<T><<<blocks, threads, 0, st>>>(*p);
+      sar_exec_simt_kernel<T><<<blocks, threads, simt_smem_bytes(table_ops(*p)), st>>>(*p);
     }
     return (int)cudaGetLastError();
   });
@@ -349,8 +349,9 @@ int sar_cuda_emulated_fit(int dtype, int path, int threads, int stages, int num_
       return threads == simta::kThreadsShared
                  ? (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sar_emul_simta_kernel<T, simta::kThreadsShared>, simta::kThreadsShared, 0)
                  : (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sar_emul_simta_kernel<T, simta::kThreads>, simta::kThreads, 0);
-    if (threads == 256) return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sar_emul_simt_kernel<T, 256>, 256, 0);
-    return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sar_emul_simt_kernel<T, 512>, threads <= 0 ? 512 : threads, 0);
+    const uint32_t smem = simt_smem_bytes((uint32_t)num_ops);
+    if (threads == 256) return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sar_emul_simt_kernel<T, 256>, 256, smem);
+    return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sar_emul_simt_kernel<T, 512>, threads <= 0 ? 512 : threads, smem);
   });
   return sms * per_sm;
 }
@@ -374,9 +375,9 @@ int sar_cuda_launch_emulated(const SarLaunchParams* params, int n, int path, int
   return with_dtype(E.common.dtype, [&](auto tag) -> int {
     using T = decltype(tag);
     void* args[] = {(void*)&E, (void*)&blocks_per_rank};
+    uint32_t nops = 0;
+    for (int r = 0; r < n; ++r) nops = table_ops(params[r]) > nops ? table_ops(params[r]) : nops;
     if (path == SAR_PATH_TMA) {
-      uint32_t nops = 0;
-      for (int r = 0; r < n; ++r) nops = table_ops(params[r]) > nops ? table_ops(params[r]) : nops;
       const uint32_t smem = tma::smem_bytes(nops, tma::stages_in_use(E.common.stages));
       int e = allow_smem(sar_emul_tma_kernel<T>);
       if (e) return e;
@@ -389,7 +390,7 @@ int sar_cuda_launch_emulated(const SarLaunchParams* params, int n, int path, int
                  : (int)cudaLaunchCooperativeKernel((void*)sar_emul_simta_kernel<T, simta::kThreads>, dim3(n * blocks_per_rank), dim3(simta::kThreads), args, 0, st);
     if (threads <= 0) threads = 512;
     return (int)cudaLaunchCooperativeKernel(threads == 256 ? (void*)sar_emul_simt_kernel<T, 256> : (void*)sar_emul_simt_kernel<T, 512>,
-                                            dim3(n * blocks_per_rank), dim3(threads), args, 0, st);
+                                            dim3(n * blocks_per_rank), dim3(threads), args, simt_smem_bytes(nops), st);
   });
 }
 

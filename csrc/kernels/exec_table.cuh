@@ -995,15 +995,17 @@ __device__ void leave_collective(const SarLaunchParams& P, const WaitCtx& w, uin
   if (P.trace) P.trace[1] = globaltimer();
 }
 
+// `table_mem`: shared memory for the rank's table (simt_smem_bytes of its ops).  With room for the largest table in
+// every block, 32-thread blocks would fit an SM ten at a time instead of sixteen.
+__host__ __device__ __forceinline__ constexpr uint32_t simt_smem_bytes(uint32_t nops) { return nops * (uint32_t)(sizeof(OpGeom) + sizeof(SarOp)); }
 template <typename T>
-__device__ void run_rank_simt(const SarLaunchParams& P, uint32_t block, uint32_t nblocks) {
+__device__ void run_rank_simt(const SarLaunchParams& P, uint32_t block, uint32_t nblocks, unsigned char* table_mem) {
   __shared__ TableGeom G;
-  __shared__ SarOp s_ops[SAR_MAX_OPS];
-  __shared__ OpGeom s_op[SAR_MAX_OPS];
   __shared__ Item s_item;
   __shared__ int s_state;   // 1: item ready, 0: table exhausted, -1: a wait failed
   WaitCtx w = enter_collective(P, block);
-  resolve_table(P, G, nblocks, s_ops, s_op);
+  OpGeom* const op_mem = reinterpret_cast<OpGeom*>(table_mem);
+  resolve_table(P, G, nblocks, reinterpret_cast<SarOp*>(op_mem + table_ops(P)), op_mem);
   ItemWalker walk;
   uint32_t arrived = 1u << P.rank, gate_passed = 0;
   if (threadIdx.x == 0) {

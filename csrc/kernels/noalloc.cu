@@ -46,11 +46,12 @@ unsigned char* g_scratch[64] = {};
 template <typename T>
 __global__ void __launch_bounds__(512, 1) sar_noalloc_kernel(const SarLaunchParams* params, int blocks_per_rank) {
   __shared__ SarLaunchParams P;
+  __shared__ __align__(16) unsigned char table_mem[sar_noalloc_impl::sar_dev::simt_smem_bytes(SAR_MAX_OPS)];
   const int r = blockIdx.x / blocks_per_rank;
   for (uint32_t i = threadIdx.x; i < sizeof(SarLaunchParams) / 4; i += blockDim.x)
     reinterpret_cast<uint32_t*>(&P)[i] = reinterpret_cast<const uint32_t*>(params + r)[i];
   __syncthreads();
-  run_rank_simt<T>(P, blockIdx.x % blocks_per_rank, blocks_per_rank);
+  run_rank_simt<T>(P, blockIdx.x % blocks_per_rank, blocks_per_rank, table_mem);
 }
 
 int fail(char* err, int errlen, int code, const char* msg) {

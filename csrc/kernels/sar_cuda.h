@@ -38,8 +38,10 @@ int sar_cuda_pick_blocks(int path, uint64_t bytes);
 int sar_cuda_lone_blocks(uint64_t bytes);
 uint32_t sar_cuda_lone_tile_bytes(int path);
 uint32_t sar_cuda_default_tile_bytes(int path);
-int sar_cuda_max_emulated_blocks(int dtype, int path, int threads);   // resident blocks on the current device
-// the same for a launch of 256-thread blocks on the simta path (threads = 256), or with `stages` ring stages (0: all; bulk-copy path) and tables of at most num_ops ops
+// Blocks that can be resident together on the current device, whatever the table (the largest one takes shared memory
+// that the usual ones leave to more 32-thread blocks).
+int sar_cuda_max_emulated_blocks(int dtype, int path, int threads);
+// the same for tables of at most num_ops ops and, on the bulk-copy path, `stages` ring stages (0: all)
 int sar_cuda_emulated_fit(int dtype, int path, int threads, int stages, int num_ops);
 
 // Barrier across ranks on control channel `channel`: announces `epoch` and

@@ -122,7 +122,7 @@ static int emulated_blocks(sar_local_comm* c, const sar_program* prog, int dtype
   if (path == SAR_PATH_SIMTA || (path == SAR_PATH_SIMT && *threads <= 0)) *threads = 256;
   cudaSetDevice(c->ranks[0].dev);   // occupancy is that of the current device
   int nops = 0;
-  if (path == SAR_PATH_TMA)
+  if (path != SAR_PATH_SIMTA)
     for (int ph = 0; ph < sar_program_num_phases(prog); ++ph)
       for (int r = 0; r < c->n; ++r) nops = std::max(nops, sar_table_num_ops(sar_program_phase(prog, ph), r));
   const auto key = std::make_tuple(dtype, path, *threads, stages, nops);

@@ -444,3 +444,20 @@ def test_gating_is_decided_when_the_program_is_compiled(monkeypatch):
     for a, b in zip(rounds, rounds[1:]):
         assert max(t[a][1] for t in tr if a in t) <= min(t[b][0] for t in tr if b in t)
     comm.close()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_sixteen_small_simt_blocks_per_sm(dtype):
+    """An explicit launch of sixteen 32-thread blocks per SM (what their registers allow) is not refused for the table's
+    shared memory."""
+    from stragglar_b200 import ops
+    n, count = 4, 600_000
+    comm = ops.LocalComm(n, emulate=True)
+    blocks = torch.cuda.get_device_properties(0).multi_processor_count * 16 // n
+    xs = _inputs(n, count, dtype)
+    want = torch.stack([x.double() for x in xs]).sum(0)
+    comm.run(sc.compile_program("ring", n), xs, path="simt", blocks=blocks, threads=32, timeout_s=5.0)
+    comm.sync()
+    for x in xs:
+        torch.testing.assert_close(x.double(), want, **TOL[dtype])
+    comm.close()
