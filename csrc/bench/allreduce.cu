@@ -20,7 +20,7 @@
 // bench_common.h).  Each of <NUM_BYTES>, <ALG> and <DELAY> may be a
 // comma-separated list; the matrix then runs in one process.  An ALG entry may carry
 // options of its own, "name:key=value:...", which override the environment for that entry:
-// blocks, stages, win (store groups in flight), tile (bytes), path (run options) and copy, lanes, lane1, gate, slack, gatemin
+// blocks, stages, win (without effect), tile (bytes), path (run options) and copy, lanes, lane1, gate, slack, gatemin
 // (the STRAGGLAR_COPY / _LANES / _LANE1_EIGHTHS / _GATE / _GATE_SLACK / _GATE_MIN_BYTES lowering switches).
 #include <algorithm>
 #include <cmath>
@@ -82,7 +82,7 @@ static std::string apply_variant(const std::string& label, Options& o, std::vect
     const std::string k = parts[i].substr(0, eq), v = parts[i].substr(eq + 1);
     if (k == "blocks") o.blocks = atoi(v.c_str());
     else if (k == "stages") o.stages = atoi(v.c_str());
-    else if (k == "win") o.store_window = atoi(v.c_str());
+    else if (k == "win") { o.store_window = atoi(v.c_str()); note_store_window(parts[i].c_str()); }
     else if (k == "tile") o.tile_bytes = (uint32_t)strtoul(v.c_str(), nullptr, 10);
     else if (k == "path") o.path = path_from(v.c_str());
     else {

@@ -76,8 +76,14 @@ inline const char* path_label(int path, int mc_groups) {
 inline const char* dtype_name(int d) { return d == SAR_F32 ? "float32" : d == SAR_BF16 ? "bfloat16" : "float16"; }
 inline uint32_t dtype_size(int d) { return d == SAR_F32 ? 4 : 2; }
 
+inline void note_store_window(const char* given) {
+  fprintf(stderr, "%s is accepted and has no effect: runs that differ in it are the same run\n", given);
+}
+
 inline Options read_options() {
   Options o;
+  o.store_window = (int)env_int("STRAGGLAR_STORE_WINDOW", 0);
+  if (o.store_window > 0) note_store_window("STRAGGLAR_STORE_WINDOW");
   int visible = 0;
   CHECK_CUDA(cudaGetDeviceCount(&visible));
   o.emulate = env_int("STRAGGLAR_EMULATE", 0) != 0;
@@ -97,7 +103,6 @@ inline Options read_options() {
   o.blocks = (int)env_int("STRAGGLAR_BLOCKS", 0);
   o.threads = (int)env_int("STRAGGLAR_THREADS", 0);
   o.stages = (int)env_int("STRAGGLAR_STAGES", 0);
-  o.store_window = (int)env_int("STRAGGLAR_STORE_WINDOW", 0);
   o.tile_bytes = (uint32_t)env_int("STRAGGLAR_TILE_BYTES", 0);
   o.timeout_s = env_int("STRAGGLAR_TIMEOUT_MS", 10000) / 1000.0;
   o.warmup = (int)env_int("STRAGGLAR_WARMUP", 10);

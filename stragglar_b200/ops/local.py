@@ -154,6 +154,9 @@ class LocalComm:
         ``user_tensors`` (one per rank, any of the three dtypes, same numel) selects staged mode for a single-phase
         program: ``tensors`` then only serve as the buffers the ranks reach into; the kernel reads rank r's input
         from ``user_tensors[r]`` and writes the result back there, converting between the two dtypes."""
+        if store_window > 0:
+            import warnings
+            warnings.warn("store_window is accepted and has no effect: runs that differ in it are the same run", stacklevel=2)
         if len(tensors) != self.n:
             raise ValueError(f"need {self.n} tensors")
         t0 = tensors[0]

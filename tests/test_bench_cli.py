@@ -33,6 +33,13 @@ def test_allreduce_rejects_unknown_algorithm():
     assert p.returncode != 0 and "Invalid algorithm: tree" in p.stderr
 
 
+def test_allreduce_store_window_says_that_it_has_no_effect():
+    # said before the program looks for devices
+    p = subprocess.run([AR, "1024", "rsag", "1", "-1"], capture_output=True, text=True,
+                       env={**os.environ, "STRAGGLAR_STORE_WINDOW": "8"})
+    assert "STRAGGLAR_STORE_WINDOW" in p.stderr and "no effect" in p.stderr
+
+
 def test_reducescatter_usage():
     p = subprocess.run([RS], capture_output=True, text=True)
     assert p.returncode != 0 and "Usage:" in p.stderr and "<bufferSize> <numIters>" in p.stderr

@@ -461,3 +461,19 @@ def test_sixteen_small_simt_blocks_per_sm(dtype):
     for x in xs:
         torch.testing.assert_close(x.double(), want, **TOL[dtype])
     comm.close()
+
+
+@pytest.mark.parametrize("store_window", [3, 16])
+def test_store_window_says_that_it_has_no_effect(store_window):
+    """A sweep over it would compare identical runs: the call goes on, with a warning."""
+    from stragglar_b200 import ops
+    comm = ops.LocalComm(2, emulate=True)
+    prog = sc.compile_program("rsag", 2)
+    xs = _inputs(2, 10_001, torch.float32)
+    want = torch.stack([x.double() for x in xs]).sum(0)
+    with pytest.warns(UserWarning, match="store_window .* no effect"):
+        comm.run(prog, xs, path="tma", timeout_s=5.0, store_window=store_window)
+    comm.sync()
+    for x in xs:
+        torch.testing.assert_close(x.double(), want, **TOL[torch.float32])
+    comm.close()
