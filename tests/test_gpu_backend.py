@@ -106,13 +106,22 @@ def _lone_rank(rank, world):
             else:
                 sp.all_reduce_ex(t, average=True, comm_dtype=wire).wait()
             assert torch.equal(t, want), (count, dtype, off, wire)
+        # in place, wherever the tensor lives: one launch
+        s = sp.empty_symmetric(count, dtype=torch.float32, device=dev)
+        s.copy_(x[:count])
+        for t in (s, x[:count].clone()):
+            want, before = t.clone(), sp.launches(dev)
+            dist.all_reduce(t, op=dist.ReduceOp.AVG)
+            assert sp.launches(dev) == before + 1 and torch.equal(t, want), count
     torch.cuda.synchronize()
     assert sp.check_status(dev) == 0 and sp.check_guards(dev)
 
 
 def test_lone_rank_of_every_size():
     """A group of one: symmetric or not, aligned or not, converted or not, up to sizes whose staged launch used to need
-    more blocks than fit the device at once."""
+    more blocks than fit the device at once.  The mean of one rank is the tensor itself (rounded to the wire), so this
+    shows that the calls end, launch what they should and leave the values alone; that every element is worked on is
+    tested with another scale (test_lone_rank_scales_every_element)."""
     run_ranks(1, _lone_rank)
 
 

@@ -477,3 +477,61 @@ def test_store_window_says_that_it_has_no_effect(store_window):
     for x in xs:
         torch.testing.assert_close(x.double(), want, **TOL[torch.float32])
     comm.close()
+
+
+UNIT = {torch.float32: 2.0 ** -24, torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}   # half an ulp, relative
+
+
+@pytest.mark.parametrize("path", PATHS)
+@pytest.mark.parametrize("wire", list(UNIT))
+@pytest.mark.parametrize("user", list(UNIT))
+@pytest.mark.parametrize("offset", [0, 1])   # elements: an aligned tensor of the caller's, and one that no vector fits
+def test_staging_of_every_type_pair(user, wire, offset, path):
+    """Tiles of far more vectors than a block has threads, so that the unrolled conversions run and end raggedly: with the
+    launch shape chosen for emulated ranks and with large tiles on few blocks."""
+    from stragglar_b200 import ops
+    n, count, guard = 2, 1_000_003, 16
+    comm = ops.LocalComm(n, emulate=True)
+    prog = sc.compile_program("rsag", n)
+    for shape in ({}, {"blocks": 3, "tile_bytes": 98304}):
+        whole = [torch.full((guard + offset + count + guard,), 7.0, dtype=user, device="cuda:0") for _ in range(n)]
+        users = [w[guard + offset:guard + offset + count] for w in whole]
+        for u, x in zip(users, _inputs(n, count, torch.float32)):
+            u.copy_(x)
+        want = torch.stack([u.to(wire).double() for u in users]).sum(0) * 0.5
+        arena = [torch.full((count,), float("nan"), dtype=wire, device="cuda:0") for _ in range(n)]
+        comm.run(prog, arena, path=path, scale=0.5, timeout_s=5.0, user_tensors=users, **shape)
+        comm.sync()
+        for w, u in zip(whole, users):
+            # the sum of two values in fp32, one rounding to the wire and one to the caller's type; atol: subnormal fp16
+            torch.testing.assert_close(u.double(), want, rtol=2.0 ** -24 + UNIT[wire] + UNIT[user] + 2.0 ** -18, atol=2.0 ** -23)
+            assert (w[:guard + offset] == 7.0).all() and (w[guard + offset + count:] == 7.0).all()
+    comm.close()
+
+
+@pytest.mark.parametrize("path", PATHS)
+def test_lone_rank_scales_every_element(path):
+    """A communicator of one rank (the launch shape of a c10d group of one) halves its buffer: one product and one rounding
+    an element, so equal bits, at one block's worth, around a block per ring stage and beyond a block per SM; with nothing
+    written beside it.  Staged: rounded to the wire, halved, rounded to the wire and to the caller's type."""
+    from stragglar_b200 import ops
+    comm = ops.LocalComm(1)
+    prog = sc.compile_program("stragglar", 1)
+    guard = 64
+    for count in (1, 5, 8 * 1024 + 1, 1 << 20, 9 * (1 << 20) + 3, 34 * (1 << 20) + 1):
+        for dtype, wire in ((torch.float32, None), (torch.bfloat16, None), (torch.float16, None), (torch.float32, torch.float32),
+                            (torch.float32, torch.bfloat16), (torch.bfloat16, torch.float32), (torch.float16, torch.bfloat16)):
+            whole = torch.full((count + 2 * guard,), 7.0, dtype=dtype, device="cuda:0")
+            t = whole[guard:guard + count]
+            t.normal_(generator=torch.Generator(device="cuda:0").manual_seed(count))
+            on_wire = t if wire is None else t.to(wire)
+            want = (on_wire.float() * 0.5).to(on_wire.dtype).to(dtype)
+            if wire is None:
+                comm.run(prog, [t], path=path, scale=0.5, timeout_s=5.0)
+            else:
+                arena = torch.full((count,), float("nan"), dtype=wire, device="cuda:0")
+                comm.run(prog, [arena], path=path, scale=0.5, timeout_s=5.0, user_tensors=[t])
+            comm.sync()
+            assert torch.equal(t, want), (count, dtype, wire)
+            assert (whole[:guard] == 7.0).all() and (whole[guard + count:] == 7.0).all(), (count, dtype, wire)
+    comm.close()
