@@ -540,6 +540,9 @@ Compiled compile(const Plan& plan, const std::vector<int>& l2p_in, int n_physica
             co.local_ver = (uint8_t)ver(s.srcs[0]);
             co.post_ver = 0;
             co.push_ver = (uint8_t)(ver(s.dst) + 1);
+            // with the pre-phase in the plan every input is read before its slot is pushed to (the sum contains it);
+            // without it the non-stragglers' other chunks are not
+            if (ver(s.dst) == 0 && slot[s.dst][s.chunk].readers.empty()) co.flags |= SAR_F_UNREAD;
             ops[s.srcs[0]].push_back(co);
           } else {
             co.kind = SAR_COPY;
@@ -637,6 +640,7 @@ Compiled compile(const Plan& plan, const std::vector<int>& l2p_in, int n_physica
               m.nsrc < SAR_MAX_RANKS - 1) {
             m.src[m.nsrc] = op.src[0];
             m.src_ver[m.nsrc] = op.src_ver[0];
+            m.flags |= op.flags & SAR_F_UNREAD;
             ++m.nsrc;
             done = true;
             break;

@@ -59,6 +59,8 @@ enum SarOpKind : uint8_t { SAR_COPY = 0, SAR_REDUCE = 1, SAR_REDUCE_PUSH = 2, SA
 enum SarOpFlag : uint8_t {
   SAR_F_SCALE = 1,  // multiply the result by the launch's scale (fused AVG / pre-division)
   SAR_F_LOCAL = 2,  // REDUCE: the own slot is one of the addends
+  SAR_F_UNREAD = 4, // PUSH: nothing before it reads the input in a destination's slot, so nothing but its flag tells when a
+                    // staged launch has copied that input in (and will not write over what is pushed)
 };
 enum SarDtype : int32_t { SAR_F32 = 0, SAR_BF16 = 1, SAR_F16 = 2 };
 

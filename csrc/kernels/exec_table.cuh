@@ -552,10 +552,11 @@ __device__ bool wait_item_ready(const SarLaunchParams& P, const Item& it, const 
   // every flag the item depends on, polled together: the loads of one turn are independent (the loop is unrolled and
   // the words stay in registers), so waiting for seven peers' tiles costs one trip over the link per turn, not seven
   // (A push names the version it replaces in the destination.  Version 0 there, in staged mode, is the
-  // destination's own copy-in of that tile, and whatever is pushed into a slot contains that rank's contribution to
-  // the chunk or follows a read of it, both of which waited for that copy-in: the push is ordered after it already.)
+  // destination's own copy-in of that tile.  Where an earlier op reads it, that op has waited for the copy-in and the push
+  // is ordered after it already; where none does, SAR_F_UNREAD, the push waits itself, or the copy-in could overwrite
+  // the pushed tile and its flag.)
   const bool own_flag = op->local_ver || staged;
-  const bool zero_flag = staged && op->kind != SAR_PUSH;
+  const bool zero_flag = staged && (op->kind != SAR_PUSH || (op->flags & SAR_F_UNREAD));
   uint32_t deps = 0;
   for (int q = 0; q < nsrc; ++q) deps |= (uint32_t)(op->src_ver[q] || zero_flag) << q;
   if (!deps) {

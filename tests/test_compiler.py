@@ -268,6 +268,43 @@ def test_round_gating_on_request_is_part_of_the_program(monkeypatch):
         assert not by_default.main.gate_asked
 
 
+@pytest.mark.parametrize("prephase", [True, False])
+@pytest.mark.parametrize("alg", ["stragglar", "stragglar_a2a", "ring", "rhd", "direct", "rsag"])
+def test_pushes_to_slots_that_nothing_has_read_are_marked(alg, prephase, monkeypatch):
+    """F_UNREAD: in staged mode nothing but the push itself can wait for the copy-in of an input that no earlier op reads.
+    With the pre-phase in the same phase there is no such push."""
+    monkeypatch.setenv("STRAGGLAR_COPY", "push")
+    F_UNREAD = 4
+    for n in (2, 4, 8):
+        main = sc.compile_program(alg, n, prephase).main
+        todo = [(int(o["round"]), r, o) for r in range(n) for o in main.ranks[r].ops]
+        read, marked, pushes = set(), 0, 0
+        for rnd in sorted({t[0] for t in todo}):
+            now = [t for t in todo if t[0] == rnd]
+            for _, r, o in now:
+                if int(o["kind"]) != sc.PUSH:
+                    continue
+                pushes += 1
+                unread = any(int(o["src_ver"][q]) == 0 and (int(o["src"][q]), int(o["chunk"])) not in read
+                             for q in range(int(o["nsrc"])))
+                assert bool(int(o["flags"]) & F_UNREAD) == unread, (alg, n, rnd, r)
+                marked += unread
+            for _, r, o in now:
+                c = int(o["chunk"])
+                if int(o["kind"]) == sc.PUSH:
+                    read.add((r, c))
+                else:
+                    read.update((int(o["src"][q]), c) for q in range(int(o["nsrc"])))
+                    if int(o["kind"]) == sc.REDUCE_PUSH or int(o["flags"]) & sc.F_LOCAL:
+                        read.add((r, c))
+        if alg == "direct":        # its pre-phase is a program phase of its own, and staged mode refuses two phases
+            continue
+        if prephase or alg in ("ring", "rhd", "rsag"):
+            assert marked == 0
+        elif n > 2:
+            assert 0 < marked <= pushes
+
+
 def test_lane_split_share(monkeypatch):
     """STRAGGLAR_LANE1_EIGHTHS moves blocks between the two lanes: every split runs to the same sums and the
     default (half, alternating) is unchanged."""

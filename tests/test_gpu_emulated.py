@@ -535,3 +535,26 @@ def test_lone_rank_scales_every_element(path):
             assert torch.equal(t, want), (count, dtype, wire)
             assert (whole[:guard] == 7.0).all() and (whole[guard + count:] == 7.0).all(), (count, dtype, wire)
     comm.close()
+
+
+@pytest.mark.parametrize("path", PATHS)
+@pytest.mark.parametrize("alg", ["stragglar", "stragglar_a2a", "direct"])
+@pytest.mark.parametrize("shape", [{"blocks": 2, "tile_bytes": 2048}, {"blocks": 8, "tile_bytes": 4096}, {}])
+def test_staged_mode_without_the_prephase(alg, path, shape, monkeypatch):
+    """The non-stragglers' sum is in place, so most slots are pushed to without their input having been read: the pushed
+    tiles, and their flags, survive the copy-in of that input."""
+    from stragglar_b200 import ops
+    monkeypatch.setenv("STRAGGLAR_COPY", "push")
+    n, count = 8, 190_003
+    comm = ops.LocalComm(n, emulate=True)
+    prog = sc.compile_program(alg, n, False)
+    for rep in range(3):
+        users = _inputs(n, count, torch.float32)
+        want = torch.stack([u.double() for u in users]).sum(0)
+        _prephase(users, alg, n - 1)
+        arena = [torch.full((count,), float("nan"), device="cuda:0") for _ in range(n)]
+        comm.run(prog, arena, path=path, timeout_s=2.0, user_tensors=users, **shape)
+        comm.sync()
+        for u in users:
+            torch.testing.assert_close(u.double(), want, atol=2e-5, rtol=1e-6)
+    comm.close()
