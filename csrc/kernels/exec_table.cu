@@ -46,9 +46,9 @@ __device__ __forceinline__ void load_rank_params(const SarEmulParams& E, int r, 
 static_assert(sizeof(SarLaunchParams) % 4 == 0, "params are copied word by word");
 
 // MAX_THREADS 256: three blocks per SM at 80 registers a thread (a few spilled words), 512: one.  A block is a serial
-// chain here too, so the third one pays: 8 ranks, rhd, 64 MiB fp16 409 -> 394 us (simta 421 -> 392), 4-rank ring, 40 MB
-// 119 -> 110 us, 6 ranks, 12 MB 67.7 -> 62.6 us, against two blocks at 128 registers.  Four blocks at 64 registers with
-// half the vectors in flight: level on simt, 5 % slower on simta.
+// chain here too, so the third one pays.  simt, three blocks per SM / two / one of 512 threads: 8 ranks, rhd, 64 MiB fp16
+// 386 / 422 / 425 us, 4-rank ring, 40 MB 112 / 119 / 140 us, 6 ranks, 12 MB 65 / 72 / 74 us.  Four blocks at 64 registers
+// with half the vectors in flight: level on simt, 5 % slower on simta.
 template <typename T, int MAX_THREADS>
 __global__ void __launch_bounds__(MAX_THREADS, MAX_THREADS == 256 ? 3 : 1) sar_emul_simt_kernel(const __grid_constant__ SarEmulParams E, int blocks_per_rank) {
   __shared__ SarLaunchParams P;

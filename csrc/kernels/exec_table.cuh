@@ -191,9 +191,9 @@ __device__ __forceinline__ void record_failure(const WaitCtx& w, uint32_t code) 
   __threadfence_system();
 }
 // Pause between two polls: short when the polled words are in this device's own L2, growing to 0.4 us when other ranks'
-// polls and data share the links.  With the acquiring load in wait_word (instead of a load and a fence) and the
-// non-suspending test in the bulk-copy consumer, 8 ranks on one device: 1 MiB bf16 stragglar_a2a 45.8 -> 43.8 us,
-// 25 MiB fp32 143.5 -> 140.2 us, bf16-wire bucket 192 -> 186 us; 4-rank ring, 40 MB 115 -> 110 us.
+// polls and data share the links.  Together with the acquiring load in wait_word (instead of a load and a fence) this
+// takes 2 to 4 % off a collective of ranks on one device (1 MiB bf16 stragglar_a2a and 4-rank ring, 40 MB: 4 %, 8 ranks,
+// 25 MiB fp32: 2 %).
 __device__ __forceinline__ void poll_pause(uint32_t& ns, const WaitCtx& w, uint32_t longest = 400) {
   __nanosleep(ns);
   if (ns < (w.one_device ? 64u : longest)) ns += ns >> 1;
@@ -274,9 +274,9 @@ struct TableGeom {
 //
 // Ranks that share a device are bound by its memory rather than by their links, and there every block does everything
 // in turn (SAR_STAGE_EVERYWHERE): a split keeps half of the blocks waiting, for tiles to come in or to become final.
-// No block waits before its own share is in, so the order cannot deadlock.  8 ranks, 25 MiB fp32 buckets: 268 us
-// against 326 with half, 331 with 3/8 and 381 with a quarter of the blocks staging; bf16 on the wire: 192 us against
-// 271, 354 and 495 (5/8: 234).
+// No block waits before its own share is in, so the order cannot deadlock.  8 ranks, 25 MiB fp32 buckets: half of the
+// blocks staging takes 1.2 times as long, a quarter 1.4 times; with bf16 on the wire 5/8 takes 1.2 times, half 1.4 times
+// and a quarter 2.6 times as long.  (Every block staging: 250 us and 154 us.)
 __device__ __forceinline__ uint32_t staging_blocks(const SarLaunchParams& P, uint32_t nblocks) {
   if (!P.user_in || nblocks < 2) return 0;
   if (P.staging_blocks == SAR_STAGE_EVERYWHERE) return 0;
@@ -290,11 +290,12 @@ __host__ __device__ __forceinline__ uint32_t table_ops(const SarLaunchParams& P)
 //
 // Bound by latency, on the path of every collective: the table is fetched with one round of coalesced loads (ops and
 // round offsets together), and everything derived from it is computed by as many threads as there are ops or rounds.
-// Walking the ops in global memory with one thread instead cost a trip to L2 per op, and every later look at an op
+// Walking the ops in global memory with one thread instead costs a trip to L2 per op, and every later look at an op
 // another one, because the acquiring fences of the waits empty L1.
-// Eight ranks on one device, 4 KiB: 38 -> 19 us in the kernel (rsag, bulk-copy path), 34 -> 15 us (simt); of that the
-// fences at device scope and the flag polls kept in registers (wait_item_ready) are about half.  With the chunks worked
-// out on the host, no fence on arrival and no exit handshake (leave_collective): 19.1 -> 15.1 us, simt 14.4 -> 10.3 us.
+// Eight ranks on one device, rsag, 4 KiB: 15 us in the kernel (simt: 10 us) against 38 us (34) with the table in global
+// memory, fences at system scope, flag words in local memory, the chunks divided out by every block and the exit
+// handshake.  The table here and the fences and polls (fence_ranks, wait_item_ready) give about 10 us each, the chunks
+// from the host and the entry and exit without fences and handshake (leave_collective) 4 us.
 __device__ void resolve_table(const SarLaunchParams& P, TableGeom& G, uint32_t nblocks, SarOp* ops_mem, OpGeom* op_mem) {
   const uint32_t nrounds = P.num_rounds < SAR_MAX_ROUNDS ? P.num_rounds : SAR_MAX_ROUNDS;
   const uint32_t nops = nrounds ? table_ops(P) : 0;
@@ -526,7 +527,8 @@ __device__ __noinline__ bool wait_gate(const SarLaunchParams& P, uint32_t round,
 __device__ bool wait_item_ready(const SarLaunchParams& P, const Item& it, const WaitCtx& w, uint32_t* arrived_mask,
                                 uint32_t* gate_passed) {
   const SarOp* op = it.op;
-  if (op->kind == SAR_STAGE_IN) return true;   // the previous collective's exit barrier has released the slot
+  // the previous collective has released the slot: its exit barrier, or (ranks on one device) the end of its launch
+  if (op->kind == SAR_STAGE_IN) return true;
   if (op->kind == SAR_STAGE_OUT)
     return wait_word(P.comm.flags[P.rank] + it.fidx, P.epoch_base + it.need_ver, w, SAR_TIMEOUT_FLAG);
   // staged mode: version 0 of a tile exists once its owner has copied it in, which the tile's flag tells
@@ -583,9 +585,9 @@ __device__ bool wait_item_ready(const SarLaunchParams& P, const Item& it, const 
   }
 }
 
-// Announces a finished tile.  The caller has ordered the tile's stores before
-// this call at system scope (fence_sys after the block barrier); the flags are
-// plain system-scope stores after that fence (release pattern).
+// Announces a finished tile.  The caller has ordered the tile's stores before this call for the other ranks (fence_ranks
+// after the block barrier: system scope, or device scope when the ranks share the device); the flags are plain
+// system-scope stores after that fence (release pattern).
 __device__ __forceinline__ void publish_item(const SarLaunchParams& P, const SarOp* op, uint32_t fidx) {
   if (op->kind == SAR_STAGE_OUT) return;
   if (op->kind == SAR_STAGE_IN) { st_relaxed_sys(P.comm.flags[P.rank] + fidx, P.epoch_base); return; }   // version 0
@@ -686,7 +688,7 @@ template <int N> __device__ __forceinline__ void store_user_vec(char* p, int dty
 // A staging tile: SAR_STAGE_IN copies the caller's elements into the own slot (wire type T), SAR_STAGE_OUT copies
 // the own slot into the caller's output.  Same element type and 16-byte aligned on both sides: vector copies;
 // otherwise the elements are converted one wire vector at a time, with vector accesses on both sides where the caller's
-// side is aligned (8 ranks, 25 MiB fp32 buckets, bf16 wire, simt: 317 -> 203 us; element by element before).  `tid` of
+// side is aligned (8 ranks, 25 MiB fp32 buckets, bf16 wire, simt: 197 us; element by element 1.6 times as long).  `tid` of
 // `nth` threads work together.
 template <typename T>
 __device__ void stage_tile(const SarLaunchParams& P, const Item& it, const uint32_t tid, const uint32_t nth) {
@@ -878,7 +880,7 @@ __device__ void simt_tile(const SarLaunchParams& P, const Item& it, const uint32
       }
     } else if (nsrc == 0) {
       // a lone rank scales its buffer in place: nothing to add, so twice the vectors in flight
-      // (1 GiB fp32 with one vector at a time: 647 to 775 us, depending on the tile; now 366)
+      // (1 GiB fp32: 371 us; 647 to 775 us, depending on the tile, with one vector at a time)
       auto scaled = [&](uint4 r) {
         float f[N];
         Vec<T>::unpack(r, f);
@@ -1075,11 +1077,11 @@ struct StageDesc {
 
 // Dynamic shared memory of a block: this structure, the op table (ops_offset), and the ring of `stages` stages
 // (ring_offset).  A launch that asks for fewer than kStages stages may allocate just those.
-// Ranks on one device: a block is a serial chain (wait, load, add, store, announce) at some 27 GB/s, whatever its ring
-// holds, so two blocks with three stages each share an SM instead of one with six.  8 ranks, fp32: 25 MiB 206 -> 141 us,
-// 256 MiB 1634 -> 1137 us, a staged 25 MiB bucket 464 -> 323 us.  Since a stage is handed back as soon as it is stored
-// (run_rank_tma): 123 us at 25 MiB, against 133 with three blocks of two stages and 130 to 155 with stages of 16 or
-// 24 KiB and as many blocks as fit.
+// Ranks on one device: a block is a serial chain (wait, load, add, store, announce), whatever its ring holds, so two
+// blocks with three stages each share an SM instead of one with six.  8 ranks, fp32, two blocks of three stages / one of
+// six / three of two: 25 MiB 123 / 164 / 137 us, 256 MiB 967 / 1256 / 1037 us, a staged 25 MiB bucket 256 / 313 / 267 us,
+// with bf16 on the wire 161 / 211 / 157 us.  Stages of 16 or 24 KiB with as many blocks as fit are 5 to 25 % slower at
+// 25 MiB.
 struct Shared {
   alignas(8) uint64_t full[kStages];    // the piece's loads have landed (and its descriptor is written)
   alignas(8) uint64_t added[kStages];   // every consumer warp is done with the piece
@@ -1171,8 +1173,8 @@ __device__ __forceinline__ uint32_t pow2_ceil(uint32_t x) {
 // Converts `elems` (a multiple of 8) elements in shared memory with NT threads.  Bound by latency: four elements a
 // thread and turn (16 bytes on the 4-byte side, 8 on the 2-byte side, consecutive threads on consecutive words, so
 // without bank conflicts) and four independent turns at a time.  One type pair is chosen per piece, not per element.
-// 8 ranks, 25 MiB fp32 buckets, bf16 wire: 487 -> 421 us (eight elements a turn at a stride of 32 bytes before), and
-// 270 us with two blocks per SM.
+// 8 ranks, 25 MiB fp32 buckets, bf16 wire: eight elements a turn at a stride of 32 bytes take 16 % longer.  fp16 buckets,
+// 12.5 MiB, over a bf16 wire: 119 us, as long as bf16 buckets that need no conversion.
 template <int SDT, int DDT> __device__ __forceinline__ uint4 convert4(uint4 v) {
   float f[4];
   if constexpr (SDT == SAR_F32) {
@@ -1244,13 +1246,15 @@ __device__ __forceinline__ bool staging_converts(const SarLaunchParams& P) { ret
 //                          item's stores have completed announce it (fence + flag stores).
 // Completion of bulk stores can only be waited for, and announcing costs a fence: a
 // storer spends that time on its own item while the others keep storing, so the
-// latency of neither is on the path that loads, adds or recycles stages.  Before, one
-// consumer thread stored, handed a stage back one piece late, let three stores be in
-// flight and told a signal thread what had landed when a store left that window or the
-// pipeline ran dry.  8 ranks on one device: 256 MiB fp32 1034 -> 961 us, 25 MiB 137 ->
-// 122 us, bf16-wire bucket 179 -> 157 us, 1 MiB bf16 stragglar_a2a 39.7 -> 37.7 us;
-// 4-rank ring, 40 MB 108 -> 95 us.  (Handing stages back at once from the consumer
-// thread instead: 1001 us, but 143 us at 25 MiB.)
+// latency of neither is on the path that loads, adds or recycles stages.  That holds for
+// items that are small next to the ring: pieces go through it in order and an item's go to
+// one storer, which waits for each to be read, so while an item of at least as many pieces
+// as the ring has stages is stored the other storers have nothing to do (256 KiB tiles, 16
+// pieces, 8 ranks on one device: 977 us against 968 with 64 KiB at 256 MiB; between GPUs
+// not measured).  One consumer thread that stores, hands a stage back one piece late with
+// three stores in flight and tells a signal thread what has landed is slower, 8 ranks on
+// one device: 256 MiB fp32 by 8 %, 25 MiB by 12 %, bf16-wire bucket by 14 %, 1 MiB bf16
+// stragglar_a2a by 5 %; 4-rank ring, 40 MB by 14 %.
 template <typename T>
 __device__ void run_rank_tma(const SarLaunchParams& P, uint32_t block, uint32_t nblocks, tma::Shared& S) {
   using namespace tma;
@@ -1543,12 +1547,13 @@ __device__ void run_rank_tma(const SarLaunchParams& P, uint32_t block, uint32_t 
 }
 
 // ------------------------------------------------------- simt path, decoupled
-// The simt data path with the control work taken off the threads that move data (512 threads):
-//   warps 0-13           workers: move the tile with 16-byte loads and stores (simt_tile);
-//   warp 14, one thread  control: walks the items and waits for their operands (flags in
-//                        peer memory) one item ahead of the workers;
-//   warp 15, one thread  signal: announces finished items (system-scope fence + flag stores).
-// In run_rank_simt every tile pays, on all 512 threads, the flag wait before it and the fence
+// The simt data path with the control work taken off the threads that move data (512 threads, or 256 when ranks that
+// share a device fill it):
+//   all warps but two    workers: move the tile with 16-byte loads and stores (simt_tile);
+//   last but one, one thread  control: walks the items and waits for their operands (flags
+//                        in the slot owner's memory) one item ahead of the workers;
+//   last, one thread     signal: announces finished items (fence_ranks + flag stores).
+// In run_rank_simt every tile pays, on all threads, the flag wait before it and the fence
 // after it; here both overlap the workers' copying.  This is also the path on which
 // reductions over, and pushes to, a whole multicast group go through the switch.
 namespace simta {
@@ -1576,9 +1581,8 @@ template <int WORKERS> __device__ __forceinline__ void worker_bar() { asm volati
 }  // namespace simta
 
 // THREADS per block: all but the last two warps are workers.  A block moves one tile at a time; with 256 threads
-// several of them fit an SM and one copies while another turns over.  8 ranks on one device, rhd, 64 MiB fp16: 504 us
-// with one 512-thread block per SM, 443 us with two of 256 threads, 424 us with tiles of 256 KiB, 392 us with three
-// blocks.
+// several of them fit an SM and one copies while another turns over.  Ranks on one device, three blocks of 256 threads
+// per SM / one of 512: rhd, 8 ranks, 64 MiB fp16 393 / 409 us, 4-rank ring, 40 MB 116 / 137 us.
 template <typename T, int THREADS>
 __device__ void run_rank_simta(const SarLaunchParams& P, uint32_t block, uint32_t nblocks, simta::Shared& S) {
   using namespace simta;

@@ -114,10 +114,10 @@ static DevTable* upload(Rank& rk, const sar_table* t, int rank, char* err, int e
 // Launch shape of a collective whose ranks share one device: as many blocks per rank as can be resident together,
 // but no more than one per 16 KiB of a rank's buffer (tiles start at 2 KiB: below that the blocks find no work and
 // only lengthen the entry).  Every block is a serial chain of wait, move, announce, so bandwidth comes from their
-// number.  On the simt path 256 threads a block let three chains share an SM where 512 leave it one.
-// 8 ranks, fp32, against 4 blocks per rank: 25 MiB 742 -> 199 us, 256 MiB 7.68 -> 1.61 ms (one bulk-copy block per SM;
-// two since then, see tma::Shared); 6 ranks, simt, 12 MB 349 -> 70 us (two blocks per SM;
-// 76 us with one of 512 threads).
+// number.  On the simt paths 256 threads a block let three chains share an SM where 512 leave it one (sar_emul_simt_kernel),
+// on the bulk-copy path three ring stages two (tma::Shared).  8 ranks, fp32, against 4 blocks per rank: 25 MiB 123 us
+// against 563, 256 MiB 0.97 ms against 5.41; 6 ranks, simt, 12 MB 64 us against 230.
+// The launch is cooperative, so it starts when the whole device is free for it.
 static int emulated_blocks(sar_local_comm* c, const sar_program* prog, int dtype, int path, int* threads, int stages, uint64_t bytes) {
   if (path == SAR_PATH_SIMTA || (path == SAR_PATH_SIMT && *threads <= 0)) *threads = 256;
   cudaSetDevice(c->ranks[0].dev);   // occupancy is that of the current device
@@ -230,15 +230,17 @@ int sar_local_run(sar_local_comm* c, const sar_program* prog, void* const* bufs,
   int blocks = o->blocks > 0 ? o->blocks : sar_cuda_pick_blocks(path, count * esize);
   int threads = path == SAR_PATH_SIMT ? o->threads : 0, stages = o->stages;
   if (c->emulate && o->blocks <= 0) {
-    if (path == SAR_PATH_TMA && stages <= 0) stages = 3;   // two blocks per SM (see emulated_blocks)
+    if (path == SAR_PATH_TMA && stages <= 0) stages = 3;   // two blocks per SM (see tma::Shared)
     blocks = emulated_blocks(c, prog, dtype, path, &threads, stages, count * esize);
   }
   const bool lone = n == 1 && !c->emulate && o->blocks <= 0;
   if (lone) { blocks = sar_cuda_lone_blocks(count * esize); if (stages <= 0) stages = 6; }
   const double timeout_s = o->timeout_s > 0 ? o->timeout_s : 10.0;
   // Emulated ranks, simt and simta: tiles of up to 256 KiB, because the wait, the block barriers and the fence around
-  // a tile are not hidden behind another one (ring, 4 ranks, 40 MB: 124 us against 137 with 128 KiB; level where the
-  // blocks outnumber the tiles).  The bulk-copy ring hides them: 64 KiB.
+  // a tile are not hidden behind another one (256 / 128 / 64 KiB: ring, 4 ranks, 40 MB 112 / 113 / 120 us, simta
+  // 116 / 116 / 124 us; rhd, 8 ranks, 64 MiB fp16 386 / 386 / 402 us, simta 394 / 403 / 398 us; level where the blocks
+  // outnumber the tiles).  The bulk-copy ring hides them: 64 KiB (8 ranks, 25 MiB 124 us against 129 with 32, 128 or
+  // 256 KiB; 256 MiB 968 against 976, 977 and 1033 us with 128, 256 and 32 KiB).
   const uint32_t tile_max = o->tile_bytes ? o->tile_bytes : lone ? sar_cuda_lone_tile_bytes(path)
                           : (c->emulate && path != SAR_PATH_TMA ? (256u << 10) : sar_cuda_default_tile_bytes(path));
   std::vector<bool> delayed(n, false);
@@ -267,7 +269,7 @@ int sar_local_run(sar_local_comm* c, const sar_program* prog, void* const* bufs,
     const int hint = sar_table_blocks_hint(t);
     if (o->blocks <= 0 && !c->emulate && hint > 0 && hint < pblocks) pblocks = hint;
     // Gating keeps the rounds of a matching-based schedule from contending for the ports of the switch.  Emulated
-    // ranks have no ports, only the hand-shake's cost (256 MiB, 8 ranks: 1140 us gated, 1048 us free-running): they
+    // ranks have no ports, only the hand-shake's cost (256 MiB, 8 ranks: 1061 us gated, 964 us free-running): they
     // are gated when that was asked for (STRAGGLAR_GATE, read when the program is compiled).
     const bool gate_wanted = !c->emulate || sar_table_gate_asked(t);
     const bool gated = gate_wanted && sar_table_gate_rounds(t) && count * esize >= sar_gate_min_bytes();

@@ -24,7 +24,8 @@ struct sar_run_opts {
   float scale;            // fused multiplier of the result
   int timed;              // 1: bracket every rank's work with events after a device-side start barrier
   int trace_rounds;       // 1: keep per-round statistics of this run (see sar_local_round_trace)
-  int stages;             // bulk-copy path: shared-memory ring stages per block (<= 0: all six)
+  int stages;             // bulk-copy path: shared-memory ring stages per block (<= 0: three for emulated ranks whose
+                          // blocks are chosen here, all six for a lone rank, else what the table asks for or all six)
   int store_window;       // accepted and without effect: a storer waits for every piece to be read, so a window on its
                           // unfinished stores (3, 8 or 16 pieces) changed nothing measurable, and testing it cost 1 %
   // Staged mode (single-phase programs): bufs[r] only serves as the buffer peers can reach; rank r's input is read

@@ -151,6 +151,9 @@ class LocalComm:
         """Enqueue ``program`` in place on ``tensors`` (one per rank).  ``trace_rounds`` keeps per-round
         statistics of this run for :meth:`round_trace`.
 
+        Emulated ranks take the whole device by default: the cooperative launch begins when no other kernel is running
+        and none runs beside it.  ``blocks`` (per rank; 4 leaves most of the device free) bounds that.
+
         ``user_tensors`` (one per rank, any of the three dtypes, same numel) selects staged mode for a single-phase
         program: ``tensors`` then only serve as the buffers the ranks reach into; the kernel reads rank r's input
         from ``user_tensors[r]`` and writes the result back there, converting between the two dtypes."""
