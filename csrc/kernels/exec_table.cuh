@@ -971,7 +971,10 @@ __device__ __forceinline__ WaitCtx enter_collective(const SarLaunchParams& P, ui
 __device__ void leave_collective(const SarLaunchParams& P, const WaitCtx& w, uint32_t nblocks) {
   SarCtrl* me = P.comm.ctrl[P.rank];
   if (w.one_device) {
+    // round gating: the counting of this rank's items, by whichever thread, comes before the last block's reset of it
+    if (P.gate_rounds) __threadfence();
     if (atomicAdd(&me->blocks_done, 1u) + 1u != nblocks) return;
+    if (P.gate_rounds) __threadfence();
     me->blocks_done = 0;
     me->items_done = 0;
     me->announced = 0;

@@ -558,3 +558,25 @@ def test_staged_mode_without_the_prephase(alg, path, shape, monkeypatch):
         for u in users:
             torch.testing.assert_close(u.double(), want, atol=2e-5, rtol=1e-6)
     comm.close()
+
+
+@pytest.mark.parametrize("path", PATHS)
+def test_gated_runs_one_after_another_on_the_whole_device(path, monkeypatch):
+    """The last block of a launch resets the counters of the gate for the next one: back to back, with every block that
+    fits, no announcement is lost."""
+    from stragglar_b200 import ops
+    monkeypatch.setenv("STRAGGLAR_GATE", "all")
+    monkeypatch.setenv("STRAGGLAR_GATE_MIN_BYTES", "0")
+    monkeypatch.setenv("STRAGGLAR_GATE_SLACK", "3")
+    n, count = 8, 200_003
+    comm = ops.LocalComm(n, emulate=True)
+    prog = sc.compile_program("stragglar", n)
+    xs = _inputs(n, count, torch.float32)
+    want = torch.stack([x.double() for x in xs]).mean(0)
+    for _ in range(100):
+        comm.run(prog, xs, path=path, scale=1.0 / n, timeout_s=2.0)
+    comm.sync()
+    # each run after the first averages n equal values: a sum of eight, one rounding or less a run
+    for x in xs:
+        torch.testing.assert_close(x.double(), want, rtol=100 * 8 * 2.0 ** -24, atol=1e-5)
+    comm.close()
